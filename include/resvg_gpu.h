@@ -145,17 +145,17 @@ void rgpu_scene_free(rgpu_scene *scene);
 
 /* Tuning knobs of the raster kernels (chosen by the autotuner). */
 typedef struct rgpu_tuning {
-    uint32_t band_rows;          /* pixel rows per raster work item: 0 (auto), 1, 2, 4 or 8 */
-    uint32_t pixels_per_thread;  /* consecutive pixels per raster thread: 0 (auto), 4, 8 or 16 */
+    uint32_t band_rows;          /* 0, 1, 2, 4 or 8; kept, but chooses nothing: work items are single rows */
+    uint32_t pixels_per_thread;  /* pixels per raster thread (a warp's row piece holds 32 times as many):
+                                  * 0 (auto), 4, 8 or 16 */
     uint32_t reserved;
 } rgpu_tuning;
 int rgpu_set_tuning(const rgpu_tuning *t);
 int rgpu_get_tuning(rgpu_tuning *t);
-/* Tuning table: with band_rows 0 in the tuning, each stream (a scene or an
- * internal surface) takes the band rows of the first entry whose max_width
- * and max_draws are at least its width and draw count (band_rows 0 in the
- * entry: the built-in rule on the width).  The autotuner fills it per
- * (canvas-size bucket, path-count bucket) (resvg_gb300.batch.autotune_table). */
+/* Tuning table: band rows per (stream width, stream draws) bucket, the first
+ * entry that holds both.  Kept and returned as set; like the tuning's band_rows
+ * it chooses nothing, as the raster kernel's work items are single rows
+ * (resvg_gb300.batch.autotune_table fills it). */
 typedef struct rgpu_tuning_entry {
     uint32_t max_width, max_draws, band_rows, reserved;
 } rgpu_tuning_entry;
@@ -173,16 +173,16 @@ int rgpu_autotune(const resvg_render_tree *const *trees, const resvg_transform *
 
 /* Failure detection (no counterpart in the reference, whose only limits are
  * defensive skips: crates/resvg/src/render.rs:108-109, filter/mod.rs:343-354).
- * The raster kernel's producer/consumer hand-offs wait at most `rounds`
- * try_wait rounds (0 = the default, 4,194,304, about a second); a wait that
+ * The raster kernel waits for its commands at most `rounds` try_wait rounds
+ * (0 = the default, 4,194,304, about a second); a wait that
  * runs out makes the render return RGPU_ERR_DEVICE_FAULT with the pixmap
  * partly rendered, and the next render starts clean.  Applies to launches made
  * afterwards (a prepared scene's captured graph keeps the value it was
  * captured with). */
 int rgpu_set_wait_limit(uint32_t rounds);
 /* Test hooks of the failure paths, for the library's own tests:
- * rgpu_test_withhold_window(1) makes the first raster CTA withhold its first
- * window, so that hand-off's bounded wait must run out (no GPU fault is made);
+ * rgpu_test_withhold_window(1) makes the first raster CTA's warps not ask for
+ * their first commands, so that bounded wait must run out (no GPU fault is made);
  * rgpu_test_fail_allocations(n) makes the library's next n device or pinned
  * host allocations fail as if memory were exhausted (RGPU_ERR_OUT_OF_MEMORY,
  * the pixmap untouched). */

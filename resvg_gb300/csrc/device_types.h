@@ -28,7 +28,7 @@ struct alignas(16) GradRec {
     uint32_t n;          // number of t_values / factors / biases
     float fr0, fr1, cdx, cdy;  // two-point conical parameters (unit space)
     uint32_t _pad[3];
-    float t[kMaxGradStops];
+    float t[kMaxGradStops];  // NaN from the n-th on: no position is >= NaN
     struct Row {
         float f[4];      // colour = t * f + b (16-byte rows: one vector load each)
         float b[4];
@@ -149,12 +149,12 @@ struct LayerRec {
 };
 
 enum CmdOp : uint32_t {
-    CMD_FILL = 0,         // a = draw
+    CMD_FILL = 0,         // a = draw, b = its paint, the bits of f = its gradient or ~0
     CMD_PUSH = 1,         // a = layer, b = init (0 transparent, 1 opaque black, 2 the layer's surface)
     CMD_POP_COMPOSITE = 2,// a = popped layer, b = blend, f = opacity
     CMD_POP_CLIP = 3,     // a = popped layer: mask = 255 - alpha, applied to the new top
     CMD_POP_MASK = 4,     // a = popped layer, b = 0 luminance / 1 alpha
-    CMD_APPLY_REGION = 5, // a = draw: top *= coverage(draw)
+    CMD_APPLY_REGION = 5, // as CMD_FILL: top *= coverage(draw)
     CMD_CLEAR = 6,        // top = transparent
     CMD_END = 7,
     CMD_HAIR = 8          // a = hairline draw (HairRec): anti-aliased hairline stroke
@@ -165,10 +165,9 @@ struct Cmd {
     float f;
 };
 
-// One unit of raster work: a band of output rows [band*band_rows, +band_rows)
-// and the x range [x0, x1) of one stream.
+// One unit of raster work: the pixels [x0, x1) of one row of one stream.
 struct WorkItem {
-    uint32_t stream, band;
+    uint32_t stream, row;
     int32_t x0, x1;
 };
 
@@ -180,13 +179,14 @@ struct StreamRec {
     int32_t out_w, out_h;          // target surface size
     uint32_t out_stride;           // bytes per row
     uint64_t out_ptr;              // device pointer of the target surface
-    uint32_t band_rows, nbands;    // band height and count
-    uint32_t bin_off;              // dense (band, draw) counters for this stream
+    uint32_t task_off;             // first task of the event kernel: 32 draws of one row each
+    uint32_t bin_off;              // slots (row, draw) of this stream: bin_off + row * draw_cnt + draw - draw_off
     uint32_t max_depth;            // layer-stack depth needed
     int32_t surface;               // internal surface rendered into (filter content), or -1
     uint32_t level;                // dependency level: content streams render before their parents
-    uint32_t fill_off, fill_cnt;   // this stream's fill / region commands (indices into its commands)
+    uint32_t row_w;                // widest work item, a power of two: 64 .. kRasterMaxRow
 };
+constexpr uint32_t kRasterMaxRow = 512;
 
 
 // An anti-aliased hairline stroke (tiny-skia scan/hairline_aa.rs): its line

@@ -10,6 +10,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cmath>
+#include <limits>
 #include <cstring>
 #include <thread>
 
@@ -159,6 +160,7 @@ bool make_grad(const Shader &sh, GradRec &g) {
         if (n > (uint32_t)kMaxGradStops) return false;  // more stops than the device record holds
         g.n = n;
     }
+    for (uint32_t k = g.n; k < (uint32_t)kMaxGradStops; k++) g.t[k] = std::numeric_limits<float>::quiet_NaN();
     // device pixel -> unit space
     Xf inv;
     if (!invert(sh.ts, &inv)) return false;

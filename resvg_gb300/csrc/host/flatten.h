@@ -91,7 +91,6 @@ struct SceneBuild {
     std::vector<PatternReq> patterns;
     std::vector<HairRec> hairs;       // anti-aliased hairline strokes
     std::vector<HairSpan> hair_spans;
-    std::vector<uint32_t> fill_cmds;  // per stream: its fill / region command indices (plan_scene)
     std::vector<uint8_t> verbs;
     std::vector<float> pts;
     std::vector<StrokeJob> stroke_jobs;  // paths stroked on the device (their draws carry DRAW_STROKED)

@@ -104,16 +104,18 @@ struct HostBuf {
 };
 
 struct Tuning {
-    uint32_t band_rows = 0;  // 0: automatic (the table, else a rule on the stream width)
-    uint32_t px = 0;         // pixels per thread: 0 automatic, else 4/8/16
-    std::vector<rgpu_tuning_entry> table;  // band rows by (stream width, stream draws) bucket
+    // kept for the callers that set them: work items are single rows, so band
+    // rows and their table choose nothing
+    uint32_t band_rows = 0;
+    std::vector<rgpu_tuning_entry> table;
+    uint32_t px = 0;         // pixels per thread (row pieces of 32 px pixels): 0 automatic, else 4/8/16
 };
 
 struct Buffers {
     DevBuf verbs, pts, draws, paints, grads, layers, cmds, streams, items;
     DevBuf tpts, segs, seg_counts, seg_offsets, scan_scratch, totals;
     DevBuf edges, edge_draw, bin_counts, bin_offsets, bins;
-    DevBuf stack, span_ovf, run_ovf, err, counter, fill_cmds;
+    DevBuf stack, err, counter, headers, events;
     DevBuf hairs, hair_spans;
     // device stroking: jobs, outlines, builder scratch, segment scratch,
     // per-job status, per-draw sizes and bases
@@ -125,7 +127,7 @@ struct Buffers {
     void release() {
         DevBuf *all[] = {&verbs, &pts, &draws, &paints, &grads, &layers, &cmds, &streams, &items, &tpts, &segs,
                          &seg_counts, &seg_offsets, &scan_scratch, &totals, &edges, &edge_draw, &bin_counts,
-                         &bin_offsets, &bins, &stack, &span_ovf, &run_ovf, &err, &counter, &fill_cmds, &plane, &hairs, &hair_spans,
+                         &bin_offsets, &bins, &stack, &err, &counter, &headers, &events, &plane, &hairs, &hair_spans,
                          &sjobs, &sverbs, &spts, &sscr_verbs, &sscr_pts, &ssegs, &sstatus, &dsizes, &dbases,
                          &sdash, &sdverbs, &sdpts, &smsegs, &smpts, &smoves};
         for (DevBuf *b : all) b->release();
@@ -158,17 +160,15 @@ constexpr uint32_t kPipeMinScenes = 64;
 constexpr uint32_t kPipeChunks = 8;
 
 // A flattened submission with its work decomposition.
-constexpr uint32_t kSpanOvf = 64;  // spans one sub-scanline of one draw may hold in the raster kernel
-
 struct Plan {
     SceneBuild sb;
     std::vector<WorkItem> items;
     std::vector<uint32_t> level_off, level_cnt;  // work items per dependency level
-    uint32_t px = 8;
-    uint64_t nbins = 0;
+    uint32_t row_w = 64;    // widest work-item row
+    uint64_t nbins = 0;      // (row, draw) slots
+    uint64_t ntasks = 0;     // of the event kernel
     uint32_t max_depth = 1;
     uint32_t grid = 1;
-    uint32_t run_cap = 0;              // alpha-run overflow entries per (draw, row) pair
     uint32_t nedges = 0, nbinned = 0;  // known after the first (sizing) run
     // segment slots and transformed points: the build's own counts, or with
     // device-stroked paths the device's totals (known after the sizing run)
@@ -301,22 +301,27 @@ int upload(HostBuf &staging, DevBuf &d, const std::vector<T> &v, size_t &stage_o
     return RGPU_OK;
 }
 
-uint32_t pick_px(const SceneBuild &sb, const Tuning &tu) {
-    if (tu.px) return tu.px;
-    int32_t maxw = 0;
-    for (auto &s : sb.streams) maxw = std::max(maxw, s.out_w);
-    return maxw <= 512 ? 4 : (maxw <= 1024 ? 8 : 16);
-}
-uint32_t pick_bh(int32_t w, uint32_t draws, uint32_t px, const Tuning &tu) {
-    if (tu.band_rows) return tu.band_rows;
-    for (const auto &e : tu.table)
-        if ((uint32_t)w <= e.max_width && draws <= e.max_draws) {
-            if (e.band_rows) return e.band_rows;
-            break;
-        }
-    uint32_t bh = 1;
-    while (bh < 8 && (256 / (bh * 2)) * px >= (uint32_t)w) bh *= 2;
-    return bh;
+// The row width of a dependency level's work items (one warp each): the widest
+// that still gives every SM about ten warps.  Wide rows cost least per pixel (a
+// draw is set up once per item), but an item is a serial chain, so too few of
+// them leave the SMs idle: 512 pixels against 128 measured 8.8 against 11.4 ms
+// on 1024^2 pixels (2048 items), 0.55 against 0.50 ms on 512^2 (512 items) and
+// 1.01 against 0.82 ms on 301 x 333.  1024 pixels were never the fastest.
+constexpr uint64_t kMinItems = 1536;
+uint32_t pick_row_w(const SceneBuild &sb, uint32_t level, const Tuning &tu) {
+    if (tu.px) return 32 * tu.px;
+    uint32_t w = 512;
+    for (; w > 64; w /= 2) {
+        uint64_t n = 0;
+        bool wide = false;  // some row is wider than half of w
+        for (const StreamRec &st : sb.streams)
+            if (st.level == level) {
+                n += (uint64_t)st.out_h * ((st.out_w + w - 1) / w);
+                wide = wide || (uint32_t)st.out_w > w / 2;
+            }
+        if (n >= kMinItems && wide) break;
+    }
+    return w;
 }
 
 // Host-side work decomposition of a flattened submission.
@@ -424,25 +429,28 @@ int plan_scene(Context &c, Plan &p) {
         int r = layout_strokes(p);
         if (r) return r;
     }
-    p.px = pick_px(sb, c.tuning);
+    p.row_w = 64;
     p.items.clear();
-    p.nbins = 0;
+    // the raster kernel finds a fill's paint and gradient through its command
+    for (Cmd &cmd : sb.cmds)
+        if (cmd.op == CMD_FILL || cmd.op == CMD_APPLY_REGION) {
+            cmd.b = sb.draws[cmd.a].paint;
+            const PaintRec &pr = sb.paints[cmd.b];
+            const uint32_t g = pr.kind == 1 ? pr.grad : 0xFFFFFFFFu;
+            std::memcpy(&cmd.f, &g, 4);
+        }
+    p.nbins = p.ntasks = 0;
     p.max_depth = 1;
-    sb.fill_cmds.clear();
+    std::vector<uint32_t> level_w(sb.max_level + 1);
+    for (uint32_t lv = 0; lv <= sb.max_level; lv++) level_w[lv] = pick_row_w(sb, lv, c.tuning);
     for (uint32_t si = 0; si < sb.streams.size(); si++) {
         StreamRec &st = sb.streams[si];
-        // the raster kernel's phase-A windows take the stream's fill commands in order
-        st.fill_off = (uint32_t)sb.fill_cmds.size();
-        for (uint32_t ci = 0; ci < st.cmd_cnt; ci++) {
-            const uint32_t op = sb.cmds[st.cmd_off + ci].op;
-            if (op == CMD_FILL || op == CMD_APPLY_REGION) sb.fill_cmds.push_back(ci);
-        }
-        st.fill_cnt = (uint32_t)sb.fill_cmds.size() - st.fill_off;
-        uint32_t bh = pick_bh(st.out_w, st.draw_cnt, p.px, c.tuning);
-        st.band_rows = bh;
-        st.nbands = (uint32_t)((st.out_h + (int32_t)bh - 1) / (int32_t)bh);
+        st.row_w = level_w[st.level];
+        p.row_w = std::max(p.row_w, st.row_w);
         st.bin_off = (uint32_t)p.nbins;
-        p.nbins += (uint64_t)st.nbands * st.draw_cnt;
+        p.nbins += (uint64_t)st.out_h * st.draw_cnt;
+        st.task_off = (uint32_t)p.ntasks;
+        p.ntasks += (uint64_t)st.out_h * ((st.draw_cnt + 31) / 32);
         p.max_depth = std::max(p.max_depth, st.max_depth + 1);
     }
     p.level_off.assign(sb.max_level + 1, 0);
@@ -452,10 +460,12 @@ int plan_scene(Context &c, Plan &p) {
         for (uint32_t si = 0; si < sb.streams.size(); si++) {
             const StreamRec &st = sb.streams[si];
             if (st.level != lv) continue;
-            int32_t cw = (int32_t)((256 / st.band_rows) * p.px);
-            for (uint32_t b = 0; b < st.nbands; b++)
+            // rows wider than row_w in pieces of about equal width
+            const int32_t np = (st.out_w + (int32_t)st.row_w - 1) / (int32_t)st.row_w;
+            const int32_t cw = ((st.out_w + np - 1) / np + 31) & ~31;
+            for (uint32_t y = 0; y < (uint32_t)st.out_h; y++)
                 for (int32_t x0 = 0; x0 < st.out_w; x0 += cw)
-                    p.items.push_back(WorkItem{si, b, x0, std::min(x0 + cw, st.out_w)});
+                    p.items.push_back(WorkItem{si, y, x0, std::min(x0 + cw, st.out_w)});
         }
         p.level_cnt[lv] = (uint32_t)p.items.size() - p.level_off[lv];
         // the persistent kernel takes items in order: heaviest first (draws x
@@ -463,18 +473,13 @@ int plan_scene(Context &c, Plan &p) {
         // a launch
         auto cost = [&](const WorkItem &it) {
             const StreamRec &st = sb.streams[it.stream];
-            return (uint64_t)st.draw_cnt * (uint64_t)(it.x1 - it.x0) * st.band_rows;
+            return (uint64_t)st.draw_cnt * (uint64_t)(it.x1 - it.x0);
         };
         std::stable_sort(p.items.begin() + p.level_off[lv], p.items.end(),
                          [&](const WorkItem &a, const WorkItem &b) { return cost(a) > cost(b); });
     }
-    if (p.nbins > 0xF0000000ull) { set_error("too many (band, draw) bins"); return RGPU_ERR_CAPACITY; }
-    // a pair's runs cover at most its work item's width, one entry per pixel
-    // step, or two per aliased span (kSpanOvf spans a scanline at most)
-    uint32_t item_w = 0;
-    for (const auto &st : sb.streams) item_w = std::max(item_w, (256 / st.band_rows) * p.px);
-    p.run_cap = std::max(item_w, 2 * kSpanOvf) + 2;
-    uint32_t per_sm = (uint32_t)raster_max_blocks_per_sm((int)p.px);
+    if (p.nbins > 0xF0000000ull) { set_error("too many (row, draw) slots"); return RGPU_ERR_CAPACITY; }
+    uint32_t per_sm = (uint32_t)raster_max_blocks_per_sm(p.row_w);
     p.grid = std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)p.items.size(), (uint32_t)c.sms * per_sm));
     return RGPU_OK;
 }
@@ -687,7 +692,7 @@ int upload_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, HostBuf *stagin
                    rup(sb.layers.size() * sizeof(LayerRec)) + rup(sb.cmds.size() * sizeof(Cmd)) +
                    rup(sb.streams.size() * sizeof(StreamRec)) + rup(p.items.size() * sizeof(WorkItem)) +
                    rup(sb.hairs.size() * sizeof(HairRec)) + rup(sb.hair_spans.size() * sizeof(HairSpan)) +
-                   rup(sb.fill_cmds.size() * 4) + rup(sb.stroke_jobs.size() * sizeof(StrokeJob)) +
+                   rup(sb.stroke_jobs.size() * sizeof(StrokeJob)) +
                    rup(sb.dashes.size() * 4) + 4096;
     CK(staging.ensure(stage));
     size_t off = 0;
@@ -703,7 +708,6 @@ int upload_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, HostBuf *stagin
     if ((r = upload(staging, b.items, p.items, off, s))) return r;
     if ((r = upload(staging, b.hairs, sb.hairs, off, s))) return r;
     if ((r = upload(staging, b.hair_spans, sb.hair_spans, off, s))) return r;
-    if ((r = upload(staging, b.fill_cmds, sb.fill_cmds, off, s))) return r;
     if ((r = upload(staging, b.sjobs, sb.stroke_jobs, off, s))) return r;
     if ((r = upload(staging, b.sdash, sb.dashes, off, s))) return r;
     if ((r = ensure_stroke_buffers(b, p))) return r;
@@ -716,10 +720,8 @@ int upload_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, HostBuf *stagin
     CK(b.scan_scratch.ensure(scan_scratch_words(std::max<uint64_t>({p.nsegs + 1, p.nbins + 1, sb.draws.size() + 1})) * 4));
     CK(b.bin_counts.ensure((p.nbins + 1) * 4));
     CK(b.bin_offsets.ensure((p.nbins + 1) * 4));
-    size_t stack_words = (size_t)p.max_depth * raster_threads() * p.px;
-    CK(b.stack.ensure((size_t)p.grid * stack_words * 4));
-    CK(b.span_ovf.ensure((size_t)p.grid * raster_threads() * kSpanOvf * 8));
-    CK(b.run_ovf.ensure((size_t)p.grid * raster_window_buffers() * raster_max_pairs() * p.run_cap * 8));
+    CK(b.headers.ensure((p.nbins + 1) * 4));
+    CK(b.stack.ensure((size_t)p.grid * raster_warps() * p.max_depth * p.row_w * 4));
     CK(b.err.ensure(16));
     CK(b.counter.ensure(4 * (sb.max_level + 1)));
     return RGPU_OK;
@@ -768,15 +770,25 @@ int enqueue_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, RasterTimer *t
         uint32_t tot = 0;
         CK(cudaMemcpyAsync(&tot, totals + 1, 4, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
+        // lists are placed by 32-bit bin offsets and slots
+        if ((uint64_t)tot + p.nbins >= 0xFFFFFFFFull) {
+            set_error("the submission's rows hold too many edges: render fewer scenes at a time");
+            return RGPU_ERR_CAPACITY;
+        }
         p.nbinned = tot;
-        CK(b.bins.ensure(std::max<uint32_t>(tot, 1) * sizeof(EdgeRec)));
+        CK(b.bins.ensure(std::max<uint32_t>(tot, 1) * 4ull));
+        CK(b.events.ensure(((uint64_t)tot + p.nbins + 1) * 16));
         p.sized = true;
     }
     CK(cudaMemsetAsync(b.bin_counts.p, 0, (p.nbins + 1) * 4, s));
     CK(cudaMemsetAsync(b.err.p, 0, 4, s));
     CK(launch_bin(true, b.edges.as<EdgeRec>(), b.edge_draw.as<uint32_t>(), nedges, b.draws.as<DrawRec>(),
                   b.streams.as<StreamRec>(), b.bin_counts.as<uint32_t>(), b.bin_offsets.as<uint32_t>(), p.nbinned,
-                  b.err.as<uint32_t>(), b.bins.as<EdgeRec>(), s));
+                  b.err.as<uint32_t>(), b.bins.as<uint32_t>(), s));
+    CK(launch_events(b.streams.as<StreamRec>(), (uint32_t)sb.streams.size(), (uint32_t)p.ntasks, b.draws.as<DrawRec>(),
+                     b.edges.as<EdgeRec>(), b.bins.as<uint32_t>(), b.bin_offsets.as<uint32_t>(),
+                     b.bin_counts.as<uint32_t>(), b.headers.as<uint32_t>(), b.events.as<uint32_t>(),
+                     b.err.as<uint32_t>(), s));
     CK(cudaMemsetAsync(b.counter.p, 0, 4 * (sb.max_level + 1), s));
     for (const auto &st : sb.streams)
         if (st.surface >= 0) CK(cudaMemsetAsync(b.surf[st.surface].p, 0, (size_t)st.out_w * st.out_h * 4, s));
@@ -789,12 +801,12 @@ int enqueue_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, RasterTimer *t
         const bool timed = tm && p.level_cnt[lv] && tm->used < RasterTimer::kPairs;
         if (timed) CK(cudaEventRecord(tm->start[tm->used], s));
         if (p.level_cnt[lv])
-            CK(launch_raster((int)p.px, p.grid, p.max_depth, b.streams.as<StreamRec>(),
+            CK(launch_raster(p.row_w, p.grid, p.max_depth, b.streams.as<StreamRec>(),
                              b.items.as<WorkItem>() + p.level_off[lv], p.level_cnt[lv], b.counter.as<uint32_t>() + lv,
-                             b.cmds.as<Cmd>(), b.fill_cmds.as<uint32_t>(), b.draws.as<DrawRec>(), b.paints.as<PaintRec>(), b.grads.as<GradRec>(),
-                             b.layers.as<LayerRec>(), b.bins.as<EdgeRec>(), b.bin_offsets.as<uint32_t>(),
-                             b.bin_counts.as<uint32_t>(), b.stack.as<uint32_t>(), b.span_ovf.as<int2>(), kSpanOvf,
-                             b.run_ovf.as<int2>(), p.run_cap, b.hairs.as<HairRec>(), b.hair_spans.as<HairSpan>(), b.err.as<uint32_t>(), s));
+                             b.cmds.as<Cmd>(), b.draws.as<DrawRec>(), b.paints.as<PaintRec>(), b.grads.as<GradRec>(),
+                             b.layers.as<LayerRec>(), b.bin_offsets.as<uint32_t>(), b.headers.as<uint32_t>(),
+                             b.events.as<uint32_t>(), b.stack.as<uint32_t>(), b.hairs.as<HairRec>(),
+                             b.hair_spans.as<HairSpan>(), b.err.as<uint32_t>(), s));
         if (timed) CK(cudaEventRecord(tm->stop[tm->used++], s));
         for (const auto &q : sb.patterns) {
             if (q.level != lv) continue;
@@ -819,7 +831,7 @@ int enqueue_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, RasterTimer *t
     }
     g_stats.draws += ndraws;
     g_stats.work_items += p.items.size();
-    g_stats.kernel_launches += 13;
+    g_stats.kernel_launches += 14;
     return RGPU_OK;
 }
 
@@ -1278,8 +1290,8 @@ int rgpu_scene_info(const rgpu_scene *sc, rgpu_scene_stats *st) {
     st->binned_edges = p.nbinned;
     st->work_items = p.items.size();
     st->grid = p.grid;
-    st->pixels_per_thread = p.px;
-    st->kernel_launches = 13;
+    st->pixels_per_thread = p.row_w / 32;
+    st->kernel_launches = 14;
     uint64_t px = 0;
     for (auto &s : p.sb.streams) px += (uint64_t)s.out_w * s.out_h;
     st->output_pixels = px;

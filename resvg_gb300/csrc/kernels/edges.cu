@@ -1,5 +1,5 @@
 // Geometry kernels: per-draw setup, per-segment edge building, exclusive scans
-// and row-band binning.
+// and row binning.
 //
 // Pipeline for one submission (all draws of all streams):
 //   k_draw_setup   thread/draw:    transform points, bounds, scan ranges
@@ -9,9 +9,10 @@
 //   scan           exclusive prefix sum -> edge offsets
 //   k_edges<true>  thread/segment: write line edges (edge_builder.rs)
 //   k_draw_edges   thread/draw:    edge range; paths with < 2 edges are dropped
-//   k_bin<false>   thread/edge:    count (band, draw) bin sizes
+//   k_bin<false>   thread/edge:    count (row, draw) bin sizes
 //   scan           -> bin offsets
-//   k_bin<true>    thread/edge:    copy edges into their bands
+//   k_bin<true>    thread/edge:    list the edge in its rows' bins
+//   k_events       events.cu:      the coverage events of every (row, draw)
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "edge_build.cuh"
@@ -191,7 +192,7 @@ __global__ void k_draw_edges(DrawRec *draws, uint32_t ndraws, const uint32_t *se
 template <bool SCATTER>
 __global__ void k_bin(const EdgeRec *edges, const uint32_t *edge_draw, uint32_t nedges, const DrawRec *draws,
                       const StreamRec *streams, uint32_t *bin_counts, const uint32_t *bin_offsets, uint32_t bin_cap,
-                      uint32_t *err, EdgeRec *bins) {
+                      uint32_t *err, uint32_t *bins) {
     uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
     if (e >= nedges) return;
     uint32_t d = edge_draw[e];
@@ -202,19 +203,15 @@ __global__ void k_bin(const EdgeRec *edges, const uint32_t *edge_draw, uint32_t 
     int32_t last_y = er.first_y + (er.hw >> 8);
     int32_t y0 = max(er.first_y, dr.start_y), y1 = min(last_y, dr.stop_y - 1);
     if (y1 < y0) return;
-    int32_t r0 = (y0 >> dr.shift) + dr.oy, r1 = (y1 >> dr.shift) + dr.oy;
-    int32_t bh = (int32_t)st.band_rows;
-    int32_t b0 = r0 >= 0 ? r0 / bh : -((-r0 + bh - 1) / bh);
-    int32_t b1 = r1 >= 0 ? r1 / bh : -((-r1 + bh - 1) / bh);
-    b0 = max(b0, 0);
-    b1 = min(b1, (int32_t)st.nbands - 1);
+    // every row the edge has a (sub)scanline in
+    const int32_t b0 = max((y0 >> dr.shift) + dr.oy, 0), b1 = min((y1 >> dr.shift) + dr.oy, st.out_h - 1);
     uint32_t ld = d - st.draw_off;
     for (int32_t b = b0; b <= b1; b++) {
         uint32_t slot = st.bin_off + (uint32_t)b * st.draw_cnt + ld;
         uint32_t k = atomicAdd(&bin_counts[slot], 1u);
         if (SCATTER) {
             uint32_t pos = bin_offsets[slot] + k;
-            if (pos < bin_cap) bins[pos] = er;
+            if (pos < bin_cap) bins[pos] = e;
             else atomicOr(err, 1u);
         }
     }
@@ -263,16 +260,17 @@ __global__ void k_scan_reduce(const uint32_t *in, uint64_t n, uint32_t *block_su
 }
 __global__ void k_scan_blocks(uint32_t *block_sums, uint32_t nblocks, uint32_t *total_out) {
     __shared__ uint32_t sh[32];
-    uint32_t carry = 0;
+    uint64_t carry = 0;
     for (uint32_t base = 0; base < nblocks; base += SCAN_T) {
         uint32_t i = base + threadIdx.x;
         uint32_t v = i < nblocks ? block_sums[i] : 0;
         uint32_t tot;
         uint32_t ex = block_exclusive(v, sh, &tot);
-        if (i < nblocks) block_sums[i] = carry + ex;
+        if (i < nblocks) block_sums[i] = (uint32_t)carry + ex;
         carry += tot;
     }
-    if (threadIdx.x == 0) *total_out = carry;
+    // a total that does not fit is reported as 2^32 - 1
+    if (threadIdx.x == 0) *total_out = (uint32_t)min(carry, (uint64_t)0xFFFFFFFFu);
 }
 __global__ void k_scan_down(const uint32_t *in, uint64_t n, const uint32_t *block_sums, uint32_t *out) {
     __shared__ uint32_t sh[32];
@@ -325,7 +323,7 @@ cudaError_t launch_draw_edges(DrawRec *draws, uint32_t ndraws, const uint32_t *s
 }
 cudaError_t launch_bin(bool scatter, const EdgeRec *edges, const uint32_t *edge_draw, uint32_t nedges,
                        const DrawRec *draws, const StreamRec *streams, uint32_t *bin_counts,
-                       const uint32_t *bin_offsets, uint32_t bin_cap, uint32_t *err, EdgeRec *bins, cudaStream_t s) {
+                       const uint32_t *bin_offsets, uint32_t bin_cap, uint32_t *err, uint32_t *bins, cudaStream_t s) {
     if (!nedges) return cudaSuccess;
     if (scatter)
         k_bin<true><<<blocks_for(nedges, 256), 256, 0, s>>>(edges, edge_draw, nedges, draws, streams, bin_counts,

@@ -48,23 +48,31 @@ cudaError_t launch_edges(bool emit, const SegRec *segs, uint32_t nsegs, const Dr
 cudaError_t launch_draw_edges(DrawRec *draws, uint32_t ndraws, const uint32_t *seg_offsets, cudaStream_t s);
 cudaError_t launch_bin(bool scatter, const EdgeRec *edges, const uint32_t *edge_draw, uint32_t nedges,
                        const DrawRec *draws, const StreamRec *streams, uint32_t *bin_counts,
-                       const uint32_t *bin_offsets, uint32_t bin_cap, uint32_t *err, EdgeRec *bins, cudaStream_t s);
+                       const uint32_t *bin_offsets, uint32_t bin_cap, uint32_t *err, uint32_t *bins, cudaStream_t s);
 size_t scan_scratch_words(uint64_t n);
 cudaError_t launch_exclusive_scan(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *scratch, uint32_t *total,
                                   cudaStream_t s);
 
+// events.cu: the coverage events of every (row, draw); headers: one word per
+// slot, events: 4 words per binned edge and per slot (events.cuh).  A task is
+// 32 draws of one row of a stream (StreamRec::task_off).
+cudaError_t launch_events(const StreamRec *streams, uint32_t nstreams, uint32_t ntasks, const DrawRec *draws,
+                          const EdgeRec *edges, const uint32_t *bins, const uint32_t *bin_offsets,
+                          const uint32_t *bin_counts, uint32_t *headers, uint32_t *events, uint32_t *err,
+                          cudaStream_t s);
+
 // raster.cu
 cudaError_t raster_init();
-size_t raster_smem_bytes();
-size_t raster_stack_words_per_cta(int px);
-int raster_threads();
-cudaError_t launch_raster(int px, uint32_t grid, uint32_t stack_depth, const StreamRec *streams, const WorkItem *items, uint32_t nitems,
-                          uint32_t *item_counter, const Cmd *cmds, const uint32_t *fill_cmds, const DrawRec *draws, const PaintRec *paints,
-                          const GradRec *grads, const LayerRec *layers, const EdgeRec *bins,
-                          const uint32_t *bin_offsets, const uint32_t *bin_counts, uint32_t *stack, int2 *span_ovf,
-                          uint32_t ovf_cap, int2 *run_ovf, uint32_t run_ovf_cap, const HairRec *hairs, const HairSpan *hair_spans, uint32_t *err,
+int raster_warps();  // warps per CTA; each takes work items of its own
+// row_w: the widest StreamRec::row_w of the launch.  stack: per warp,
+// stack_depth rows of row_w pixels.
+cudaError_t launch_raster(uint32_t row_w, uint32_t grid, uint32_t stack_depth, const StreamRec *streams,
+                          const WorkItem *items, uint32_t nitems, uint32_t *item_counter, const Cmd *cmds,
+                          const DrawRec *draws, const PaintRec *paints, const GradRec *grads, const LayerRec *layers,
+                          const uint32_t *bin_offsets, const uint32_t *headers, const uint32_t *events,
+                          uint32_t *stack, const HairRec *hairs, const HairSpan *hair_spans, uint32_t *err,
                           cudaStream_t s);
-int raster_max_blocks_per_sm(int px);
+int raster_max_blocks_per_sm(uint32_t row_w);
 // Failure-detection controls of the raster kernel: the try_wait rounds after
 // which a producer/consumer hand-off is declared stuck (0 = the default), and
 // a test hook that withholds the first window of CTA 0 so that wait must run
@@ -72,8 +80,6 @@ int raster_max_blocks_per_sm(int px);
 void raster_set_wait_limit(uint32_t rounds);
 uint32_t raster_wait_limit();
 void raster_set_withhold(bool on);
-int raster_max_pairs();  // (draw, row) pairs of one phase-A window
-int raster_window_buffers();  // phase-A window buffers per CTA (each with its own run-overflow area)
 
 // filters.cu
 cudaError_t filter_color_space(uint32_t *img, size_t n, bool to_linear, cudaStream_t s);

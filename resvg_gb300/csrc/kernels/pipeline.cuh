@@ -295,7 +295,12 @@ __device__ __forceinline__ void gradient_eval_lowp(const PaintRec &pr, const Gra
 // Two u16 lanes per register (r | b << 16, g | a << 16): every lane value of
 // the lowp source-over path stays <= 255 * 255 + 255, so lanes never carry into
 // each other and div255 = (v + 255) >> 8 runs on both at once.
-__device__ __forceinline__ uint32_t div255_2(uint32_t v) { return ((v + 0x00FF00FFu) >> 8) & 0x00FF00FFu; }
+// (Bytes 1 and 3 of the sum are the two results: one byte permute.)
+__device__ __forceinline__ uint32_t div255_2(uint32_t v) { return __byte_perm(v + 0x00FF00FFu, 0u, 0x4341); }
+// the lane pairs (r, b) and (g, a) of a pixel, and the pixel of two pairs
+__device__ __forceinline__ uint32_t pair_rb(uint32_t p) { return p & 0x00FF00FFu; }
+__device__ __forceinline__ uint32_t pair_ga(uint32_t p) { return __byte_perm(p, 0u, 0x4341); }
+__device__ __forceinline__ uint32_t from_pairs(uint32_t rb, uint32_t ga) { return __byte_perm(rb, ga, 0x6240); }
 
 // lowp gradient colour as two lane pairs (same arithmetic as gradient_eval_lowp).
 __device__ __forceinline__ void gradient_eval_lowp2(const PaintRec &pr, const GradRec &g, int32_t px, int32_t py,
@@ -313,11 +318,81 @@ __device__ __forceinline__ void gradient_eval_lowp2(const PaintRec &pr, const Gr
     }
 }
 
-__device__ __forceinline__ float4 unpack_f(uint32_t p) {
-    return make_float4((float)ch(p, 0) * kInv255, (float)ch(p, 1) * kInv255, (float)ch(p, 2) * kInv255,
-                       (float)ch(p, 3) * kInv255);
+// One pixel of a lowp colour (lane pairs rb, ga) drawn with coverage cov (0 ..
+// 255): lowp_over source-over, the colour scaled by the coverage; lowp_source
+// an opaque source, interpolated by the coverage.  Coverages 0 and 255 need no
+// branch: div255(v * 255) is v, so they give the pixel and the colour exactly.
+// The reference's coverage scale, (cov / 255) * 255 + 0.5 truncated, is cov
+// itself for every value.
+__device__ __forceinline__ uint32_t lowp_over(uint32_t rb, uint32_t ga, uint32_t cov, uint32_t dst) {
+    rb = div255_2(rb * cov);
+    ga = div255_2(ga * cov);
+    const uint32_t inv = 255u - (ga >> 16);
+    rb += div255_2(pair_rb(dst) * inv);
+    ga += div255_2(pair_ga(dst) * inv);
+    return from_pairs(rb, ga);
 }
-__device__ __forceinline__ uint32_t pack_f(float4 o) { return pack(unnorm(o.x), unnorm(o.y), unnorm(o.z), unnorm(o.w)); }
+__device__ __forceinline__ uint32_t lowp_source(uint32_t rb, uint32_t ga, uint32_t cov, uint32_t dst) {
+    const uint32_t inv = 255u - cov;
+    return from_pairs(div255_2(pair_rb(dst) * inv + rb * cov), div255_2(pair_ga(dst) * inv + ga * cov));
+}
+
+// Conversions between bytes and floats without the conversion unit (a quarter
+// of the arithmetic rate or less): a byte as the low mantissa bits of 2^23 is
+// 2^23 + byte, and adding 2^23 rounds a value in [0, 255] to the nearest even
+// integer in the low bits, as a conversion would.  Two channels per instruction.
+constexpr float kTwo23 = 8388608.0f;
+// Two float sums per instruction.  There is no two-float product here: the
+// assembler was seen to fuse mul.rn.f32x2 with a following add.rn.f32x2 into
+// one rounding, --fmad=false notwithstanding, so products stay scalar.
+__device__ __forceinline__ float2 as_float2(unsigned long long r) {
+    return make_float2(__uint_as_float((uint32_t)r), __uint_as_float((uint32_t)(r >> 32)));
+}
+__device__ __forceinline__ unsigned long long as_u64(float2 v) {
+    return (unsigned long long)__float_as_uint(v.x) | (unsigned long long)__float_as_uint(v.y) << 32;
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(as_u64(a)), "l"(as_u64(b)));
+    return as_float2(r);
+}
+__device__ __forceinline__ float2 add2_rz(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rz.f32x2 %0, %1, %2;" : "=l"(r) : "l"(as_u64(a)), "l"(as_u64(b)));
+    return as_float2(r);
+}
+__device__ __forceinline__ float two23_byte(uint32_t p, int i) {
+    return __uint_as_float(__byte_perm(p, 0x4B000000u, 0x7540 | i));
+}
+__device__ __forceinline__ float4 unpack_f(uint32_t p) {
+    const float2 off = make_float2(-kTwo23, -kTwo23);
+    const float2 a = add2(make_float2(two23_byte(p, 0), two23_byte(p, 1)), off);
+    const float2 b = add2(make_float2(two23_byte(p, 2), two23_byte(p, 3)), off);
+    return make_float4(a.x * kInv255, a.y * kInv255, b.x * kInv255, b.y * kInv255);
+}
+__device__ __forceinline__ uint32_t pack_f(float4 o) {
+    const float2 off = make_float2(kTwo23, kTwo23);
+    const float2 a = add2(make_float2(__saturatef(o.x) * 255.0f, __saturatef(o.y) * 255.0f), off);
+    const float2 b = add2(make_float2(__saturatef(o.z) * 255.0f, __saturatef(o.w) * 255.0f), off);
+    const uint32_t lo = __byte_perm(__float_as_uint(a.x), __float_as_uint(a.y), 0x0040);
+    const uint32_t hi = __byte_perm(__float_as_uint(b.x), __float_as_uint(b.y), 0x0040);
+    return __byte_perm(lo, hi, 0x5410);
+}
+// The lowp store of a gradient colour: channels clamped to [0, 1], then v * 255
+// + 0.5 truncated (2^23 added towards zero leaves the integer in the low byte),
+// as the bits 0x4B0000nn of the four floats.
+__device__ __forceinline__ uint4 lowp_bits(float r, float g, float b, float a) {
+    const float2 half = make_float2(0.5f, 0.5f), off = make_float2(kTwo23, kTwo23);
+    const float2 x = add2_rz(add2(make_float2(__saturatef(r) * 255.0f, __saturatef(g) * 255.0f), half), off);
+    const float2 y = add2_rz(add2(make_float2(__saturatef(b) * 255.0f, __saturatef(a) * 255.0f), half), off);
+    return make_uint4(__float_as_uint(x.x), __float_as_uint(x.y), __float_as_uint(y.x), __float_as_uint(y.y));
+}
+// c / 255 correctly rounded for c = 0 .. 255 (one Newton correction of the
+// product with 1 / 255; checked for all 256 values)
+__device__ __forceinline__ float byte_over_255(float c) {
+    const float q = c * kInv255;
+    return __fmaf_rn(__fmaf_rn(-q, 255.0f, c), kInv255, q);
+}
 
 // shade_pixel for the paints and blend modes off the inline fast path.
 __device__ __forceinline__ uint32_t shade_pixel_slow(const PaintRec &pr, const GradRec *grad, int32_t lx,
@@ -387,7 +462,6 @@ __device__ __forceinline__ uint32_t shade_pixel(const PaintRec &pr, const GradRe
         return pack(pr.memset_rgba[0], pr.memset_rgba[1], pr.memset_rgba[2], pr.memset_rgba[3]);
     const uint32_t blend = pr.blend;
     if ((pr.flags & PAINT_LOWP) && blend == RGPU_BLEND_SOURCE_OVER) {
-        // lowp source-over (pre-scaled by coverage), two lanes per register
         uint32_t rb, ga;
         if (pr.kind != 0) gradient_eval_lowp2(pr, *grad, lx, ly, rb, ga);
         else {
@@ -396,14 +470,7 @@ __device__ __forceinline__ uint32_t shade_pixel(const PaintRec &pr, const GradRe
             rb = __byte_perm(w0, w1, 0x5410);
             ga = __byte_perm(w0, w1, 0x7632);
         }
-        if (cov != 255) {
-            rb = div255_2(rb * cov);
-            ga = div255_2(ga * cov);
-        }
-        const uint32_t inv = 255u - (ga >> 16);
-        rb += div255_2((dst & 0x00FF00FFu) * inv);
-        ga += div255_2(((dst >> 8) & 0x00FF00FFu) * inv);
-        return (rb & 0x00FF00FFu) | ((ga & 0x00FF00FFu) << 8);
+        return lowp_over(rb, ga, cov, dst);
     }
     return shade_pixel_slow(pr, grad, lx, ly, cov, dst);
 }
@@ -411,7 +478,9 @@ __device__ __forceinline__ uint32_t shade_pixel(const PaintRec &pr, const GradRe
 // draw_pixmap of one pixel: highp pattern (already at the right pixel),
 // opacity scale, blend, store.
 __device__ __forceinline__ uint32_t composite_pixel(uint32_t src, uint32_t dst, float opacity, uint32_t blend) {
-    if (blend == RGPU_BLEND_DESTINATION) return dst;
+    // a transparent source over any pixel is that pixel (every byte survives
+    // the way to float and back)
+    if (blend == RGPU_BLEND_DESTINATION || (src == 0u && blend == RGPU_BLEND_SOURCE_OVER)) return dst;
     float4 s = unpack_f(src);
     if (opacity != 1.0f) s = make_float4(s.x * opacity, s.y * opacity, s.z * opacity, s.w * opacity);
     return pack_f(blend4(blend, s, unpack_f(dst)));
@@ -419,16 +488,17 @@ __device__ __forceinline__ uint32_t composite_pixel(uint32_t src, uint32_t dst, 
 
 // Pixmap::apply_mask (lowp): every channel *= m / 255 via div255.
 __device__ __forceinline__ uint32_t mask_pixel(uint32_t p, uint32_t m) {
-    return pack(div255(ch(p, 0) * m), div255(ch(p, 1) * m), div255(ch(p, 2) * m), div255(ch(p, 3) * m));
+    return from_pairs(div255_2(pair_rb(p) * m), div255_2(pair_ga(p) * m));
 }
 
 // Mask::from_pixmap value for one pixel.
 __device__ __forceinline__ uint32_t mask_value(uint32_t p, bool luminance) {
     uint32_t a8 = ch(p, 3);
     if (!luminance) return a8;
-    float r = (float)ch(p, 0) / 255.0f, g = (float)ch(p, 1) / 255.0f, b = (float)ch(p, 2) / 255.0f;
-    float a = (float)a8 / 255.0f;
-    if (a8 != 0) { r = __fdiv_rn(r, a); g = __fdiv_rn(g, a); b = __fdiv_rn(b, a); }
+    if (a8 == 0) return 0;  // the luminance is scaled by the alpha
+    float r = byte_over_255(two23_byte(p, 0) - kTwo23), g = byte_over_255(two23_byte(p, 1) - kTwo23);
+    float b = byte_over_255(two23_byte(p, 2) - kTwo23), a = byte_over_255((float)a8);
+    if (a8 != 255) { r = __fdiv_rn(r, a); g = __fdiv_rn(g, a); b = __fdiv_rn(b, a); }
     // Rec. 709 luma coefficients (tiny-skia mask.rs from_pixmap)
     float luma = r * 0.2126f + g * 0.7152f + b * 0.0722f;
     float v = ceilf(fminf(fmaxf((luma * a) * 255.0f, 0.0f), 255.0f));
