@@ -1,9 +1,9 @@
 // Device edge builder: per path segment, the fixed-point edges Skia's edge
 // builder produces (tiny-skia 0.12.0 edge.rs / edge_builder.rs / edge_clipper.rs /
-// path_geometry.rs).  Each thread owns one segment and runs the same f32/f64
-// and 16.16 fixed-point arithmetic serially; curve edges are expanded into their
-// forward-differenced line pieces up front instead of lazily inside the scan
-// loop, which yields the identical sequence of line edges.
+// path_geometry.rs).  A thread chops and clips one segment into monotonic pieces
+// with the same f32/f64 arithmetic; a warp then expands each piece into its
+// forward-differenced 16.16 fixed-point lines up front, instead of lazily inside
+// the scan loop, which yields the identical line edges.
 #pragma once
 #include <stdint.h>
 #include "../device_types.h"
@@ -139,6 +139,7 @@ __device__ __forceinline__ int chop_quad_at_x_extrema(const Pt *src, Pt *dst) {
 
 // ---- fixed point
 __device__ __forceinline__ int32_t wadd(int32_t a, int32_t b) { return (int32_t)((uint32_t)a + (uint32_t)b); }
+__device__ __forceinline__ int32_t wsub(int32_t a, int32_t b) { return (int32_t)((uint32_t)a - (uint32_t)b); }
 __device__ __forceinline__ int32_t lsh(int32_t v, int s) { return (int32_t)((uint32_t)v << s); }
 __device__ __forceinline__ int32_t fdot6_round(int32_t n) { return (n + 32) >> 6; }
 __device__ __forceinline__ int32_t fdot6_to_fdot16(int32_t v) { return lsh(v, 10); }
@@ -182,137 +183,154 @@ __device__ __forceinline__ int32_t cubic_delta_from_line(int32_t a, int32_t b, i
     return max(abs(one_third), abs(two_third));
 }
 
-// Sink receiving the line edges of one segment (counting or writing).
-struct EdgeSink {
-    EdgeRec *out;    // null: count only
+// A monotonic piece of a segment after chopping and clipping: a line, quad or
+// cubic (kind 1, 2, 3) whose edges a warp makes together (expand_piece).
+struct Piece {
+    Pt p[4];
+    uint32_t kind;
+};
+// One segment's pieces: at most 3 x 3 monotonic parts of a clipped cubic, each
+// with a vertical line on either side.
+constexpr int kMaxPieces = 27;
+struct PieceSink {
+    Piece *out;
     uint32_t n;
-    uint32_t cap;
-    __device__ __forceinline__ void put(const LineE &e, int winding) {
-        if (out && n < cap) {
-            EdgeRec r;
-            r.x = e.x; r.dx = e.dx; r.first_y = e.first_y;
-            r.hw = ((e.last_y - e.first_y) << 8) | (winding & 0xff);
-            out[n] = r;
+    __device__ __forceinline__ void put(uint32_t kind, const Pt *p) {
+        if (n < (uint32_t)kMaxPieces) {
+            out[n].kind = kind;
+            for (uint32_t i = 0; i <= kind; i++) out[n].p[i] = p[i];
         }
         n++;
     }
 };
+__device__ __forceinline__ void push_line(PieceSink &s, Pt p0, Pt p1) {
+    const Pt p[2] = {p0, p1};
+    s.put(1, p);
+}
+__device__ __forceinline__ void push_quad(PieceSink &s, const Pt *p) { s.put(2, p); }
+__device__ __forceinline__ void push_cubic(PieceSink &s, const Pt *p) { s.put(3, p); }
 
-__device__ __forceinline__ void push_line(EdgeSink &s, Pt p0, Pt p1, int shift) {
-    float scale = (float)(1 << (shift + 6));
-    int32_t x0 = sat_i32(p0.x * scale), y0 = sat_i32(p0.y * scale);
-    int32_t x1 = sat_i32(p1.x * scale), y1 = sat_i32(p1.y * scale);
-    int w = 1;
-    if (y0 > y1) { int32_t t = x0; x0 = x1; x1 = t; t = y0; y0 = y1; y1 = t; w = -1; }
-    int32_t top = fdot6_round(y0), bottom = fdot6_round(y1);
-    if (top == bottom) return;
-    int32_t slope = fdot6_div(x1 - x0, y1 - y0);
-    int32_t dy = compute_dy(top, y0);
-    LineE e;
-    e.x = fdot6_to_fdot16(x0 + fdot16_mul(slope, dy));
-    e.dx = slope;
-    e.first_y = top;
-    e.last_y = bottom - 1;
-    s.put(e, w);
+__device__ __forceinline__ int32_t warp_prefix(int32_t v) {  // inclusive, wrapping
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int32_t t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v = wadd(v, t);
+    }
+    return v;
 }
 
-__device__ __noinline__ void push_quad(EdgeSink &s, const Pt *pts, int shift) {
-    float scale = (float)(1 << (shift + 6));
-    int32_t x0 = sat_i32(pts[0].x * scale), y0 = sat_i32(pts[0].y * scale);
-    int32_t x1 = sat_i32(pts[1].x * scale), y1 = sat_i32(pts[1].y * scale);
-    int32_t x2 = sat_i32(pts[2].x * scale), y2 = sat_i32(pts[2].y * scale);
+// The line edges of one piece, by a whole warp: f(lane's edge, winding, valid)
+// once per 32 forward-difference steps.  tiny-skia steps a curve with running
+// sums of shifted differences; every step's difference is known in closed form
+// or is itself a sum, so the steps come from prefix sums (wrapping 32-bit
+// integers: the same values) and each lane makes one line, the division for its
+// slope included.  Zero-height lines are skipped as the lazy updater skips them.
+template <class F>
+__device__ __forceinline__ void expand_piece(const Piece &pc, int shift_aa, F f) {
+    const int lane = threadIdx.x & 31;
+    const float scale = (float)(1 << (shift_aa + 6));
+    int32_t x0 = sat_i32(pc.p[0].x * scale), y0 = sat_i32(pc.p[0].y * scale);
+    int32_t x1 = sat_i32(pc.p[1].x * scale), y1 = sat_i32(pc.p[1].y * scale);
     int w = 1;
-    if (y0 > y2) { int32_t t = x0; x0 = x2; x2 = t; t = y0; y0 = y2; y2 = t; w = -1; }
-    int32_t top = fdot6_round(y0), bot = fdot6_round(y2);
-    if (top == bot) return;
-    {
-        int32_t dx = (lsh(x1, 1) - x0 - x2) >> 2;
-        int32_t dy = (lsh(y1, 1) - y0 - y2) >> 2;
-        shift = diff_to_shift(dx, dy, shift);
-    }
-    if (shift == 0) shift = 1;
-    else if (shift > 6) shift = 6;
-    int count = 1 << shift;
-    int cshift = shift - 1;
-    int32_t A = lsh(x0 - x1 - x1 + x2, 9);
-    int32_t B = fdot6_to_fdot16(x1 - x0);
-    int32_t qx = fdot6_to_fdot16(x0), qdx = B + (A >> shift), qddx = A >> (shift - 1);
-    A = lsh(y0 - y1 - y1 + y2, 9);
-    B = fdot6_to_fdot16(y1 - y0);
-    int32_t qy = fdot6_to_fdot16(y0), qdy = B + (A >> shift), qddy = A >> (shift - 1);
-    int32_t lastx = fdot6_to_fdot16(x2), lasty = fdot6_to_fdot16(y2);
-    int32_t oldx = qx, oldy = qy;
-    // expand every forward-difference step; zero-height pieces are skipped as
-    // the lazy updater would skip them
-    while (count > 0) {
-        int32_t newx, newy;
-        count--;
-        if (count > 0) {
-            newx = oldx + (qdx >> cshift); qdx += qddx;
-            newy = oldy + (qdy >> cshift); qdy += qddy;
-        } else {
-            newx = lastx; newy = lasty;
+    if (pc.kind == 1) {
+        if (y0 > y1) { int32_t t = x0; x0 = x1; x1 = t; t = y0; y0 = y1; y1 = t; w = -1; }
+        const int32_t top = fdot6_round(y0), bottom = fdot6_round(y1);
+        LineE e{0, 0, 0, 0};
+        if (top != bottom) {
+            const int32_t slope = fdot6_div(x1 - x0, y1 - y0);
+            e.x = fdot6_to_fdot16(x0 + fdot16_mul(slope, compute_dy(top, y0)));
+            e.dx = slope;
+            e.first_y = top;
+            e.last_y = bottom - 1;
         }
-        LineE e;
-        if (line_update(e, oldx, oldy, newx, newy)) s.put(e, w);
-        oldx = newx; oldy = newy;
+        f(e, w, lane == 0 && top != bottom);
+        return;
     }
-}
-
-__device__ __noinline__ void push_cubic(EdgeSink &s, const Pt *pts, int shift) {
-    float scale = (float)(1 << (shift + 6));
-    int32_t x0 = sat_i32(pts[0].x * scale), y0 = sat_i32(pts[0].y * scale);
-    int32_t x1 = sat_i32(pts[1].x * scale), y1 = sat_i32(pts[1].y * scale);
-    int32_t x2 = sat_i32(pts[2].x * scale), y2 = sat_i32(pts[2].y * scale);
-    int32_t x3 = sat_i32(pts[3].x * scale), y3 = sat_i32(pts[3].y * scale);
-    int w = 1;
-    if (y0 > y3) {
-        int32_t t;
-        t = x0; x0 = x3; x3 = t; t = x1; x1 = x2; x2 = t;
-        t = y0; y0 = y3; y3 = t; t = y1; y1 = y2; y2 = t;
-        w = -1;
-    }
-    int32_t top = fdot6_round(y0), bot = fdot6_round(y3);
-    if (top == bot) return;
-    {
-        int32_t dx = cubic_delta_from_line(x0, x1, x2, x3);
-        int32_t dy = cubic_delta_from_line(y0, y1, y2, y3);
-        shift = diff_to_shift(dx, dy, 2) + 1;
-    }
-    if (shift > 6) shift = 6;
-    int up_shift = 6;
-    int down_shift = shift + up_shift - 10;
-    if (down_shift < 0) { down_shift = 0; up_shift = 10 - shift; }
-    int32_t B = lsh(3 * (x1 - x0), up_shift);
-    int32_t C = lsh(3 * (x0 - x1 - x1 + x2), up_shift);
-    int32_t D = lsh(x3 + 3 * (x1 - x2) - x0, up_shift);
-    int32_t cx = fdot6_to_fdot16(x0);
-    int32_t cdx = B + (C >> shift) + (D >> (2 * shift));
-    int32_t cddx = 2 * C + ((3 * D) >> (shift - 1));
-    int32_t cdddx = (3 * D) >> (shift - 1);
-    B = lsh(3 * (y1 - y0), up_shift);
-    C = lsh(3 * (y0 - y1 - y1 + y2), up_shift);
-    D = lsh(y3 + 3 * (y1 - y2) - y0, up_shift);
-    int32_t cy = fdot6_to_fdot16(y0);
-    int32_t cdy = B + (C >> shift) + (D >> (2 * shift));
-    int32_t cddy = 2 * C + ((3 * D) >> (shift - 1));
-    int32_t cdddy = (3 * D) >> (shift - 1);
-    int32_t lastx = fdot6_to_fdot16(x3), lasty = fdot6_to_fdot16(y3);
-    int count = -(1 << shift);
-    int32_t oldx = cx, oldy = cy;
-    while (count < 0) {
-        int32_t newx, newy;
-        count++;
-        if (count < 0) {
-            newx = oldx + (cdx >> down_shift); cdx += cddx >> shift; cddx += cdddx;
-            newy = oldy + (cdy >> down_shift); cdy += cddy >> shift; cddy += cdddy;
-        } else {
-            newx = lastx; newy = lasty;
+    int32_t x2 = sat_i32(pc.p[2].x * scale), y2 = sat_i32(pc.p[2].y * scale);
+    // running sums of the first (d) and second (a) differences of both
+    // coordinates at the 32-step chunk's start
+    int32_t oldx, oldy, lastx, lasty;
+    int shift, down;
+    int32_t dx0, dy0, ax0, ay0, aax = 0, aay = 0;
+    const bool cubic = pc.kind == 3;
+    if (!cubic) {
+        if (y0 > y2) { int32_t t = x0; x0 = x2; x2 = t; t = y0; y0 = y2; y2 = t; w = -1; }
+        if (fdot6_round(y0) == fdot6_round(y2)) return;
+        shift = diff_to_shift((lsh(x1, 1) - x0 - x2) >> 2, (lsh(y1, 1) - y0 - y2) >> 2, shift_aa);
+        if (shift == 0) shift = 1;
+        else if (shift > 6) shift = 6;
+        down = shift - 1;
+        int32_t A = lsh(x0 - x1 - x1 + x2, 9), B = fdot6_to_fdot16(x1 - x0);
+        dx0 = B + (A >> shift);
+        ax0 = A >> (shift - 1);
+        A = lsh(y0 - y1 - y1 + y2, 9);
+        B = fdot6_to_fdot16(y1 - y0);
+        dy0 = B + (A >> shift);
+        ay0 = A >> (shift - 1);
+        lastx = fdot6_to_fdot16(x2);
+        lasty = fdot6_to_fdot16(y2);
+    } else {
+        int32_t x3 = sat_i32(pc.p[3].x * scale), y3 = sat_i32(pc.p[3].y * scale);
+        if (y0 > y3) {
+            int32_t t;
+            t = x0; x0 = x3; x3 = t; t = x1; x1 = x2; x2 = t;
+            t = y0; y0 = y3; y3 = t; t = y1; y1 = y2; y2 = t;
+            w = -1;
         }
-        if (newy < oldy) newy = oldy;
-        LineE e;
-        if (line_update(e, oldx, oldy, newx, newy)) s.put(e, w);
-        oldx = newx; oldy = newy;
+        if (fdot6_round(y0) == fdot6_round(y3)) return;
+        shift = diff_to_shift(cubic_delta_from_line(x0, x1, x2, x3), cubic_delta_from_line(y0, y1, y2, y3), 2) + 1;
+        if (shift > 6) shift = 6;
+        int up = 6;
+        down = shift + up - 10;
+        if (down < 0) { down = 0; up = 10 - shift; }
+        int32_t B = lsh(3 * (x1 - x0), up), C = lsh(3 * (x0 - x1 - x1 + x2), up), D = lsh(x3 + 3 * (x1 - x2) - x0, up);
+        dx0 = B + (C >> shift) + (D >> (2 * shift));
+        aax = (3 * D) >> (shift - 1);
+        ax0 = 2 * C + aax;
+        B = lsh(3 * (y1 - y0), up);
+        C = lsh(3 * (y0 - y1 - y1 + y2), up);
+        D = lsh(y3 + 3 * (y1 - y2) - y0, up);
+        dy0 = B + (C >> shift) + (D >> (2 * shift));
+        aay = (3 * D) >> (shift - 1);
+        ay0 = 2 * C + aay;
+        lastx = fdot6_to_fdot16(x3);
+        lasty = fdot6_to_fdot16(y3);
+    }
+    oldx = fdot6_to_fdot16(x0);
+    oldy = fdot6_to_fdot16(y0);
+    const int n = 1 << shift;
+    for (int base = 0; base < n; base += 32) {
+        const int k = base + lane;
+        int32_t dx, dy;
+        if (cubic) {
+            // step k's second difference is linear in k; shifted, its sums give
+            // the first differences
+            const int32_t ax = (int32_t)((uint32_t)ax0 + (uint32_t)lane * (uint32_t)aax) >> shift;
+            const int32_t ay = (int32_t)((uint32_t)ay0 + (uint32_t)lane * (uint32_t)aay) >> shift;
+            const int32_t sx = warp_prefix(ax), sy = warp_prefix(ay);
+            dx = wadd(dx0, wsub(sx, ax)) >> down;
+            dy = max(wadd(dy0, wsub(sy, ay)) >> down, 0);  // y never steps back
+            dx0 = wadd(dx0, __shfl_sync(0xffffffffu, sx, 31));
+            dy0 = wadd(dy0, __shfl_sync(0xffffffffu, sy, 31));
+            ax0 = wadd(ax0, (int32_t)(32u * (uint32_t)aax));
+            ay0 = wadd(ay0, (int32_t)(32u * (uint32_t)aay));
+        } else {
+            dx = (int32_t)((uint32_t)dx0 + (uint32_t)k * (uint32_t)ax0) >> down;
+            dy = (int32_t)((uint32_t)dy0 + (uint32_t)k * (uint32_t)ay0) >> down;
+        }
+        const int32_t px = warp_prefix(dx), py = warp_prefix(dy);
+        const int32_t ox = wadd(oldx, wsub(px, dx)), oy = wadd(oldy, wsub(py, dy));
+        int32_t nx = wadd(oldx, px), ny = wadd(oldy, py);
+        if (k == n - 1) {
+            nx = lastx;
+            ny = cubic ? max(lasty, oy) : lasty;
+        }
+        LineE e{0, 0, 0, 0};
+        const bool ok = k < n && line_update(e, ox, oy, nx, ny);
+        f(e, w, ok);
+        oldx = wadd(oldx, __shfl_sync(0xffffffffu, px, 31));
+        oldy = wadd(oldy, __shfl_sync(0xffffffffu, py, 31));
     }
 }
 
@@ -344,7 +362,7 @@ __device__ __forceinline__ float sect_clamp_with_vertical(const Pt *src, float x
     if (a > b) { float t = a; a = b; b = t; }
     return fminf(fmaxf(y, a), b);
 }
-__device__ __noinline__ void clip_line(EdgeSink &s, Pt p0, Pt p1, const ClipR &clip, int shift) {
+__device__ __noinline__ void clip_line(PieceSink &s, Pt p0, Pt p1, const ClipR &clip) {
     Pt pts[2] = {p0, p1};
     int i0, i1;
     if (pts[0].y < pts[1].y) { i0 = 0; i1 = 1; } else { i0 = 1; i1 = 0; }
@@ -383,15 +401,15 @@ __device__ __noinline__ void clip_line(EdgeSink &s, Pt p0, Pt p1, const ClipR &c
         n = k;
     }
     if (reverse) {
-        for (int i = n - 1; i >= 0; i--) push_line(s, res[i + 1], res[i], shift);
+        for (int i = n - 1; i >= 0; i--) push_line(s, res[i + 1], res[i]);
         // emitted in the reversed point order: lines[n-i] = res[i]
     } else {
-        for (int i = 0; i < n; i++) push_line(s, res[i], res[i + 1], shift);
+        for (int i = 0; i < n; i++) push_line(s, res[i], res[i + 1]);
     }
 }
-__device__ __forceinline__ void append_vline(EdgeSink &s, float x, float y0, float y1, bool reverse, int shift) {
+__device__ __forceinline__ void append_vline(PieceSink &s, float x, float y0, float y1, bool reverse) {
     if (reverse) { float t = y0; y0 = y1; y1 = t; }
-    push_line(s, Pt{x, y0}, Pt{x, y1}, shift);
+    push_line(s, Pt{x, y0}, Pt{x, y1});
 }
 __device__ __forceinline__ bool chop_mono_quad_at(const Pt *src, float v, bool is_y, float *t) {
     float c0 = is_y ? src[0].y : src[0].x, c1 = is_y ? src[1].y : src[1].x, c2 = is_y ? src[2].y : src[2].x;
@@ -401,7 +419,7 @@ __device__ __forceinline__ bool chop_mono_quad_at(const Pt *src, float v, bool i
     if (n) { *t = roots[0]; return true; }
     return false;
 }
-__device__ __noinline__ void clip_mono_quad(EdgeSink &s, const Pt *src, const ClipR &clip, int shift) {
+__device__ __noinline__ void clip_mono_quad(PieceSink &s, const Pt *src, const ClipR &clip) {
     Pt pts[3];
     bool reverse;
     if (src[0].y > src[2].y) { pts[0] = src[2]; pts[1] = src[1]; pts[2] = src[0]; reverse = true; }
@@ -430,17 +448,17 @@ __device__ __noinline__ void clip_mono_quad(EdgeSink &s, const Pt *src, const Cl
         }
     }
     if (pts[0].x > pts[2].x) { Pt q = pts[0]; pts[0] = pts[2]; pts[2] = q; reverse = !reverse; }
-    if (pts[2].x <= clip.l) { append_vline(s, clip.l, pts[0].y, pts[2].y, reverse, shift); return; }
-    if (pts[0].x >= clip.r) { append_vline(s, clip.r, pts[0].y, pts[2].y, reverse, shift); return; }
+    if (pts[2].x <= clip.l) { append_vline(s, clip.l, pts[0].y, pts[2].y, reverse); return; }
+    if (pts[0].x >= clip.r) { append_vline(s, clip.r, pts[0].y, pts[2].y, reverse); return; }
     if (pts[0].x < clip.l) {
         if (chop_mono_quad_at(pts, clip.l, false, &t)) {
             chop_quad_at(pts, t, tmp);
-            append_vline(s, clip.l, tmp[0].y, tmp[2].y, reverse, shift);
+            append_vline(s, clip.l, tmp[0].y, tmp[2].y, reverse);
             tmp[2].x = clip.l;
             tmp[3].x = fmaxf(tmp[3].x, clip.l);
             pts[0] = tmp[2]; pts[1] = tmp[3];
         } else {
-            append_vline(s, clip.l, pts[0].y, pts[2].y, reverse, shift);
+            append_vline(s, clip.l, pts[0].y, pts[2].y, reverse);
             return;
         }
     }
@@ -451,20 +469,20 @@ __device__ __noinline__ void clip_mono_quad(EdgeSink &s, const Pt *src, const Cl
             tmp[1].x = fminf(tmp[1].x, clip.r);
             tmp[2].x = clip.r;
             if (reverse) { q[0] = tmp[2]; q[1] = tmp[1]; q[2] = tmp[0]; } else { q[0] = tmp[0]; q[1] = tmp[1]; q[2] = tmp[2]; }
-            push_quad(s, q, shift);
-            append_vline(s, clip.r, tmp[2].y, tmp[4].y, reverse, shift);
+            push_quad(s, q);
+            append_vline(s, clip.r, tmp[2].y, tmp[4].y, reverse);
         } else {
             pts[1].x = fminf(pts[1].x, clip.r);
             pts[2].x = fminf(pts[2].x, clip.r);
             if (reverse) { q[0] = pts[2]; q[1] = pts[1]; q[2] = pts[0]; } else { q[0] = pts[0]; q[1] = pts[1]; q[2] = pts[2]; }
-            push_quad(s, q, shift);
+            push_quad(s, q);
         }
     } else {
         if (reverse) { q[0] = pts[2]; q[1] = pts[1]; q[2] = pts[0]; } else { q[0] = pts[0]; q[1] = pts[1]; q[2] = pts[2]; }
-        push_quad(s, q, shift);
+        push_quad(s, q);
     }
 }
-__device__ __noinline__ void clip_quad(EdgeSink &s, const Pt *p, const ClipR &clip, int shift) {
+__device__ __noinline__ void clip_quad(PieceSink &s, const Pt *p, const ClipR &clip) {
     float t = fminf(fminf(p[0].y, p[1].y), p[2].y), b = fmaxf(fmaxf(p[0].y, p[1].y), p[2].y);
     if (!(b > clip.t && t < clip.b)) return;
     Pt mono_y[5];
@@ -472,7 +490,7 @@ __device__ __noinline__ void clip_quad(EdgeSink &s, const Pt *p, const ClipR &cl
     for (int y = 0; y <= ny; y++) {
         Pt mono_x[5];
         int nx = chop_quad_at_x_extrema(&mono_y[y * 2], mono_x);
-        for (int x = 0; x <= nx; x++) clip_mono_quad(s, &mono_x[x * 2], clip, shift);
+        for (int x = 0; x <= nx; x++) clip_mono_quad(s, &mono_x[x * 2], clip);
     }
 }
 // root of a monotonic cubic coordinate in double (bisection to convergence)
@@ -546,13 +564,13 @@ __device__ __forceinline__ void chop_mono_cubic_at(const Pt *src, float v, bool 
     float tt = mono_cubic_closest_t(is_y ? tmp + 1 : tmp, v);
     chop_cubic_at2(src, tt, dst);
 }
-__device__ __forceinline__ void emit_cubic(EdgeSink &s, const Pt *p, bool reverse, int shift) {
+__device__ __forceinline__ void emit_cubic(PieceSink &s, const Pt *p, bool reverse) {
     Pt q[4];
     if (reverse) { q[0] = p[3]; q[1] = p[2]; q[2] = p[1]; q[3] = p[0]; }
     else { q[0] = p[0]; q[1] = p[1]; q[2] = p[2]; q[3] = p[3]; }
-    push_cubic(s, q, shift);
+    push_cubic(s, q);
 }
-__device__ __noinline__ void clip_mono_cubic(EdgeSink &s, const Pt *src, const ClipR &clip, int shift) {
+__device__ __noinline__ void clip_mono_cubic(PieceSink &s, const Pt *src, const ClipR &clip) {
     Pt pts[4];
     bool reverse;
     if (src[0].y > src[3].y) { for (int i = 0; i < 4; i++) pts[i] = src[3 - i]; reverse = true; }
@@ -582,12 +600,12 @@ __device__ __noinline__ void clip_mono_cubic(EdgeSink &s, const Pt *src, const C
         q = pts[1]; pts[1] = pts[2]; pts[2] = q;
         reverse = !reverse;
     }
-    if (pts[3].x <= clip.l) { append_vline(s, clip.l, pts[0].y, pts[3].y, reverse, shift); return; }
-    if (pts[0].x >= clip.r) { append_vline(s, clip.r, pts[0].y, pts[3].y, reverse, shift); return; }
+    if (pts[3].x <= clip.l) { append_vline(s, clip.l, pts[0].y, pts[3].y, reverse); return; }
+    if (pts[0].x >= clip.r) { append_vline(s, clip.r, pts[0].y, pts[3].y, reverse); return; }
     if (pts[0].x < clip.l) {
         Pt tmp[7];
         chop_mono_cubic_at(pts, clip.l, false, tmp);
-        append_vline(s, clip.l, tmp[0].y, tmp[3].y, reverse, shift);
+        append_vline(s, clip.l, tmp[0].y, tmp[3].y, reverse);
         tmp[3].x = clip.l;
         tmp[4].x = fmaxf(tmp[4].x, clip.l);
         pts[0] = tmp[3]; pts[1] = tmp[4]; pts[2] = tmp[5];
@@ -597,48 +615,47 @@ __device__ __noinline__ void clip_mono_cubic(EdgeSink &s, const Pt *src, const C
         chop_mono_cubic_at(pts, clip.r, false, tmp);
         tmp[3].x = clip.r;
         tmp[2].x = fminf(tmp[2].x, clip.r);
-        emit_cubic(s, tmp, reverse, shift);
-        append_vline(s, clip.r, tmp[3].y, tmp[6].y, reverse, shift);
+        emit_cubic(s, tmp, reverse);
+        append_vline(s, clip.r, tmp[3].y, tmp[6].y, reverse);
     } else {
-        emit_cubic(s, pts, reverse, shift);
+        emit_cubic(s, pts, reverse);
     }
 }
-__device__ __noinline__ void clip_cubic(EdgeSink &s, const Pt *p, const ClipR &clip, int shift) {
+__device__ __noinline__ void clip_cubic(PieceSink &s, const Pt *p, const ClipR &clip) {
     float l = fminf(fminf(p[0].x, p[1].x), fminf(p[2].x, p[3].x)), r = fmaxf(fmaxf(p[0].x, p[1].x), fmaxf(p[2].x, p[3].x));
     float t = fminf(fminf(p[0].y, p[1].y), fminf(p[2].y, p[3].y)), b = fmaxf(fmaxf(p[0].y, p[1].y), fmaxf(p[2].y, p[3].y));
     if (!(b > clip.t && t < clip.b)) return;
     const float lim = (float)(1 << 22);
-    if (l < -lim || t < -lim || r > lim || b > lim) { clip_line(s, p[0], p[3], clip, shift); return; }
+    if (l < -lim || t < -lim || r > lim || b > lim) { clip_line(s, p[0], p[3], clip); return; }
     Pt mono_y[10];
     int ny = chop_cubic_at_y_extrema(p, mono_y);
     for (int y = 0; y <= ny; y++) {
         Pt mono_x[10];
         int nx = chop_cubic_at_x_extrema(&mono_y[y * 3], mono_x);
-        for (int x = 0; x <= nx; x++) clip_mono_cubic(s, &mono_x[x * 3], clip, shift);
+        for (int x = 0; x <= nx; x++) clip_mono_cubic(s, &mono_x[x * 3], clip);
     }
 }
 
-// One path segment -> line edges (EdgeBuilder::build for one PathEdge).
-__device__ __forceinline__ void build_segment(EdgeSink &s, int kind, const Pt *p, bool contained, const ClipR &clip,
-                                              int shift) {
+// One path segment -> its monotonic pieces (EdgeBuilder::build for one PathEdge).
+__device__ __forceinline__ void build_segment(PieceSink &s, int kind, const Pt *p, bool contained, const ClipR &clip) {
     if (kind == 1) {
-        if (contained) push_line(s, p[0], p[1], shift);
-        else clip_line(s, p[0], p[1], clip, shift);
+        if (contained) push_line(s, p[0], p[1]);
+        else clip_line(s, p[0], p[1], clip);
     } else if (kind == 2) {
         if (contained) {
             Pt mono[5];
             int n = chop_quad_at_y_extrema(p, mono);
-            for (int i = 0; i <= n; i++) push_quad(s, &mono[i * 2], shift);
+            for (int i = 0; i <= n; i++) push_quad(s, &mono[i * 2]);
         } else {
-            clip_quad(s, p, clip, shift);
+            clip_quad(s, p, clip);
         }
     } else if (kind == 3) {
         if (contained) {
             Pt mono[10];
             int n = chop_cubic_at_y_extrema(p, mono);
-            for (int i = 0; i <= n; i++) push_cubic(s, &mono[i * 3], shift);
+            for (int i = 0; i <= n; i++) push_cubic(s, &mono[i * 3]);
         } else {
-            clip_cubic(s, p, clip, shift);
+            clip_cubic(s, p, clip);
         }
     }
 }
