@@ -1,0 +1,47 @@
+"""The differentiable renderer's row kernels at the edges of their splits: one
+pixel to the widest canvas (lanes that scan 1 to 32 pixels), groups that the
+canvas cuts, path counts around the 32 masks read at a time, and batches large
+enough for two groups per warp, against the FP64 reference.
+
+Tolerances: the FP32 forward within 2e-4 of FP64 (values in [0, 1]); a random
+directional derivative within 1e-3 of the sum of its terms' magnitudes.
+"""
+import numpy as np
+import pytest
+
+from resvg_gb300 import soft
+
+pytestmark = pytest.mark.gpu
+
+KEYS = ("points", "colors", "stop_offsets", "stop_colors", "sigma", "opacity")
+
+
+def _arrays(scenes, w, h, paths, seed):
+    a = soft.make_scenes(seed=seed, scenes=scenes, size=max(w, h), paths=paths, min_segs=2, max_segs=5)
+    s = np.array([w, h], np.float32) / max(w, h)
+    a["width"], a["height"] = w, h
+    # a margin on every side: lines left of, right of and above the canvas too
+    a["points"] = ((a["points"] * 1.2 - 0.1 * max(w, h)) * s).astype(np.float32)
+    a["grad_line"] = (a["grad_line"] * np.tile(s, 2)).astype(np.float32)
+    return a
+
+
+@pytest.mark.parametrize("scenes,w,h,paths", [
+    (1, 1, 5, 2), (2, 31, 9, 3), (1, 32, 8, 1), (1, 33, 20, 33), (2, 65, 3, 64), (1, 127, 7, 32), (3, 255, 6, 5),
+    (1, 257, 12, 31), (1, 511, 5, 2), (1, 513, 5, 3), (1, 1024, 4, 2), (8, 256, 128, 2), (9, 250, 128, 3)])
+def test_rows_match_fp64(gpu, oracle_mod, scenes, w, h, paths):
+    import torch
+    a = _arrays(scenes, w, h, paths, seed=w + h)
+    sc = soft.Scenes(a)
+    image, blurred = soft.forward(sc)
+    im64, bl64 = oracle_mod.soft_forward(a)
+    assert np.abs(image.cpu().numpy() - im64).max() <= 2e-4
+    assert np.abs(blurred.cpu().numpy() - bl64).max() <= 2e-4
+    rng = np.random.default_rng(3)
+    target = torch.from_numpy(rng.uniform(0, 1, size=im64.shape).astype(np.float32)).cuda()
+    _, g = soft.mse(blurred, target)
+    grads = soft.backward(sc, image, g)
+    v = {k: rng.normal(size=a[k].shape) for k in KEYS}
+    terms = np.concatenate([(grads[k].double().cpu().numpy() * v[k]).ravel() for k in KEYS])
+    _, ref = oracle_mod.soft_dloss(a, target.cpu().numpy(), v)
+    assert abs(terms.sum() - ref) <= 1e-3 * np.abs(terms).sum()
