@@ -175,12 +175,18 @@ __global__ void k_box_pass(const uint32_t *src, uint32_t *dst, int len, int line
 // and moves the line through registers kIirChunk values at a time, so loads
 // and stores stay off the dependency chain.
 constexpr int kIirChunk = 16;
-__global__ void k_iir_load4(const uint32_t *img, double *planes, size_t n) {
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const uint32_t p = img[i];
+// The 256 quotients c / 255 are made once per CTA and the pixels look them up (a
+// division per value took 380 us on 2048^2 pixels: f64 runs at 2 lanes a clock
+// and SM).
+__global__ void __launch_bounds__(256) k_iir_load4(const uint32_t *img, double *planes, size_t n) {
+    __shared__ double unit[256];
+    unit[threadIdx.x] = __ddiv_rn((double)threadIdx.x, 255.0);
+    __syncthreads();
+    for (size_t i = (size_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256) {
+        const uint32_t p = img[i];
 #pragma unroll
-    for (int ch = 0; ch < 4; ch++) planes[(size_t)ch * n + i] = __ddiv_rn((double)chn(p, ch), 255.0);
+        for (int ch = 0; ch < 4; ch++) planes[(size_t)ch * n + i] = unit[chn(p, ch)];
+    }
 }
 // one line of `len` values at base[k * step]; the next chunk is loaded
 // before the current one is computed, so memory latency overlaps the chain
@@ -924,7 +930,7 @@ cudaError_t filter_iir_blur(uint32_t *img, double *buf, int w, int h, double sx,
         return iir_blur_fast(img, reinterpret_cast<float *>(buf), reinterpret_cast<float *>(buf) + 4 * n, w, h, dx,
                              dy, sx > 0.0, sy > 0.0, post, s);
     // buf holds four planes of n doubles
-    k_iir_load4<<<nblk(n, 256), 256, 0, s>>>(img, buf, n);
+    k_iir_load4<<<std::min(nblk(n, 256), 1216u), 256, 0, s>>>(img, buf, n);  // 8 CTAs on each of 152 SMs
     if (sx > 0.0) k_iir_rows4<<<nblk((size_t)4 * h, 64), 64, 0, s>>>(buf, w, h, dx, steps);
     if (sy > 0.0) k_iir_cols4<<<nblk((size_t)4 * w, 64), 64, 0, s>>>(buf, w, h, dy, steps);
     k_iir_store4<<<nblk(n, 256), 256, 0, s>>>(img, buf, n, post);
@@ -1384,8 +1390,10 @@ __device__ __forceinline__ int64_t sat_i64_d(double v) { return __double2ll_rz(v
 
 struct TurbStitch { int32_t width, height, wrap_x, wrap_y; };
 
-__device__ __forceinline__ double turb_noise2(int ch, double x, double y, const int32_t *sel, const double2 *grad,
-                                              bool stitch, const TurbStitch &st) {
+// One octave's noise of the four channels at (x, y): the lattice cell, the
+// fractions and the s-curves are the same for all of them.
+__device__ __forceinline__ void turb_noise4(double x, double y, const int32_t *sel, const double2 *grad, bool stitch,
+                                            const TurbStitch &st, double (&out)[4]) {
     double t = __dadd_rn(x, (double)kTurbPerlinN);
     int32_t bx0 = sat_i32_d(t), bx1 = (int32_t)((uint32_t)bx0 + 1u);
     const double rx0 = __dsub_rn(t, (double)sat_i64_d(t)), rx1 = __dsub_rn(rx0, 1.0);
@@ -1400,20 +1408,24 @@ __device__ __forceinline__ double turb_noise2(int ch, double x, double y, const 
     }
     bx0 &= 0xff; bx1 &= 0xff; by0 &= 0xff; by1 &= 0xff;
     const int32_t i = sel[bx0], j = sel[bx1];
-    const double2 *g = grad + ch * kTurbBLen;
+    const int32_t b00 = sel[i + by0], b10 = sel[j + by0], b01 = sel[i + by1], b11 = sel[j + by1];
     const double sx = __dmul_rn(__dmul_rn(rx0, rx0), __dsub_rn(3.0, __dmul_rn(2.0, rx0)));
     const double sy = __dmul_rn(__dmul_rn(ry0, ry0), __dsub_rn(3.0, __dmul_rn(2.0, ry0)));
-    double2 q = g[sel[i + by0]];
-    double u = __dadd_rn(__dmul_rn(rx0, q.x), __dmul_rn(ry0, q.y));
-    q = g[sel[j + by0]];
-    double v = __dadd_rn(__dmul_rn(rx1, q.x), __dmul_rn(ry0, q.y));
-    const double a = __dadd_rn(u, __dmul_rn(sx, __dsub_rn(v, u)));
-    q = g[sel[i + by1]];
-    u = __dadd_rn(__dmul_rn(rx0, q.x), __dmul_rn(ry1, q.y));
-    q = g[sel[j + by1]];
-    v = __dadd_rn(__dmul_rn(rx1, q.x), __dmul_rn(ry1, q.y));
-    const double b = __dadd_rn(u, __dmul_rn(sx, __dsub_rn(v, u)));
-    return __dadd_rn(a, __dmul_rn(sy, __dsub_rn(b, a)));
+#pragma unroll
+    for (int ch = 0; ch < 4; ch++) {
+        const double2 *g = grad + ch * kTurbBLen;
+        double2 q = g[b00];
+        double u = __dadd_rn(__dmul_rn(rx0, q.x), __dmul_rn(ry0, q.y));
+        q = g[b10];
+        double v = __dadd_rn(__dmul_rn(rx1, q.x), __dmul_rn(ry0, q.y));
+        const double a = __dadd_rn(u, __dmul_rn(sx, __dsub_rn(v, u)));
+        q = g[b01];
+        u = __dadd_rn(__dmul_rn(rx0, q.x), __dmul_rn(ry1, q.y));
+        q = g[b11];
+        v = __dadd_rn(__dmul_rn(rx1, q.x), __dmul_rn(ry1, q.y));
+        const double b = __dadd_rn(u, __dmul_rn(sx, __dsub_rn(v, u)));
+        out[ch] = __dadd_rn(a, __dmul_rn(sy, __dsub_rn(b, a)));
+    }
 }
 
 __device__ __forceinline__ bool approx_zero_ulps_d(double v) {
@@ -1457,49 +1469,59 @@ __global__ void __launch_bounds__(256) k_turbulence(uint32_t *out, int w, int h,
     }
     __syncthreads();
 
+    // the stitched frequencies do not depend on the pixel
+    double bfx = tp.bfx, bfy = tp.bfy;
+    TurbStitch st0{0, 0, 0, 0};
+    if (tp.stitch) {
+        const double tile_w = (double)w, tile_h = (double)h;
+        if (!approx_zero_ulps_d(bfx)) {
+            const double lo = __ddiv_rn(floor(__dmul_rn(tile_w, bfx)), tile_w);
+            const double hi = __ddiv_rn(ceil(__dmul_rn(tile_w, bfx)), tile_w);
+            bfx = __ddiv_rn(bfx, lo) < __ddiv_rn(hi, bfx) ? lo : hi;
+        }
+        if (!approx_zero_ulps_d(bfy)) {
+            const double lo = __ddiv_rn(floor(__dmul_rn(tile_h, bfy)), tile_h);
+            const double hi = __ddiv_rn(ceil(__dmul_rn(tile_h, bfy)), tile_h);
+            bfy = __ddiv_rn(bfy, lo) < __ddiv_rn(hi, bfy) ? lo : hi;
+        }
+        st0.width = sat_i32_d(__dadd_rn(__dmul_rn(tile_w, bfx), 0.5));
+        st0.height = sat_i32_d(__dadd_rn(__dmul_rn(tile_h, bfy), 0.5));
+    }
     const size_t n = (size_t)w * h;
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + t; idx < n; idx += (size_t)gridDim.x * blockDim.x) {
         const int x = (int)(idx % w), y = (int)(idx / w);
-        uint32_t px = 0;
-        for (int ch = 0; ch < 4; ch++) {
-            double bfx = tp.bfx, bfy = tp.bfy;
-            TurbStitch st{0, 0, 0, 0};
-            const double tile_w = (double)w, tile_h = (double)h;
+        TurbStitch st = st0;
+        if (tp.stitch) {
+            st.wrap_x = sat_i32_d(__dadd_rn(__dadd_rn(__dmul_rn((double)x, bfx), (double)kTurbPerlinN), (double)st.width));
+            st.wrap_y = sat_i32_d(__dadd_rn(__dadd_rn(__dmul_rn((double)y, bfy), (double)kTurbPerlinN), (double)st.height));
+        }
+        // a quotient by 1 is its dividend
+        const double ux = __dadd_rn((double)x, tp.ox), uy = __dadd_rn((double)y, tp.oy);
+        double vx = __dmul_rn(tp.sx == 1.0 ? ux : __ddiv_rn(ux, tp.sx), bfx);
+        double vy = __dmul_rn(tp.sy == 1.0 ? uy : __ddiv_rn(uy, tp.sy), bfy);
+        // the reference divides by 1, 2, 4, ..: products with the exact
+        // reciprocals round to the same values (2^-1023 is a double too)
+        double sum[4] = {0.0, 0.0, 0.0, 0.0}, inv = 1.0;
+        for (int o = 0; o < tp.octaves; o++) {
+            double nz[4];
+            turb_noise4(vx, vy, sel, grad, tp.stitch != 0, st, nz);
+#pragma unroll
+            for (int ch = 0; ch < 4; ch++) sum[ch] = __dadd_rn(sum[ch], __dmul_rn(tp.fractal ? nz[ch] : fabs(nz[ch]), inv));
+            vx = __dmul_rn(vx, 2.0);
+            vy = __dmul_rn(vy, 2.0);
+            inv = __dmul_rn(inv, 0.5);
             if (tp.stitch) {
-                if (!approx_zero_ulps_d(bfx)) {
-                    const double lo = __ddiv_rn(floor(__dmul_rn(tile_w, bfx)), tile_w);
-                    const double hi = __ddiv_rn(ceil(__dmul_rn(tile_w, bfx)), tile_w);
-                    bfx = __ddiv_rn(bfx, lo) < __ddiv_rn(hi, bfx) ? lo : hi;
-                }
-                if (!approx_zero_ulps_d(bfy)) {
-                    const double lo = __ddiv_rn(floor(__dmul_rn(tile_h, bfy)), tile_h);
-                    const double hi = __ddiv_rn(ceil(__dmul_rn(tile_h, bfy)), tile_h);
-                    bfy = __ddiv_rn(bfy, lo) < __ddiv_rn(hi, bfy) ? lo : hi;
-                }
-                st.width = sat_i32_d(__dadd_rn(__dmul_rn(tile_w, bfx), 0.5));
-                st.height = sat_i32_d(__dadd_rn(__dmul_rn(tile_h, bfy), 0.5));
-                st.wrap_x = sat_i32_d(__dadd_rn(__dadd_rn(__dmul_rn((double)x, bfx), (double)kTurbPerlinN),
-                                                (double)st.width));
-                st.wrap_y = sat_i32_d(__dadd_rn(__dadd_rn(__dmul_rn((double)y, bfy), (double)kTurbPerlinN),
-                                                (double)st.height));
+                st.width = (int32_t)((uint32_t)st.width * 2u);
+                st.wrap_x = (int32_t)((uint32_t)st.wrap_x * 2u - (uint32_t)kTurbPerlinN);
+                st.height = (int32_t)((uint32_t)st.height * 2u);
+                st.wrap_y = (int32_t)((uint32_t)st.wrap_y * 2u - (uint32_t)kTurbPerlinN);
             }
-            double vx = __dmul_rn(__ddiv_rn(__dadd_rn((double)x, tp.ox), tp.sx), bfx);
-            double vy = __dmul_rn(__ddiv_rn(__dadd_rn((double)y, tp.oy), tp.sy), bfy);
-            double sum = 0.0, ratio = 1.0;
-            for (int o = 0; o < tp.octaves; o++) {
-                const double nz = turb_noise2(ch, vx, vy, sel, grad, tp.stitch != 0, st);
-                sum = __dadd_rn(sum, __ddiv_rn(tp.fractal ? nz : fabs(nz), ratio));
-                vx = __dmul_rn(vx, 2.0);
-                vy = __dmul_rn(vy, 2.0);
-                ratio = __dmul_rn(ratio, 2.0);
-                if (tp.stitch) {
-                    st.width = (int32_t)((uint32_t)st.width * 2u);
-                    st.wrap_x = (int32_t)((uint32_t)st.wrap_x * 2u - (uint32_t)kTurbPerlinN);
-                    st.height = (int32_t)((uint32_t)st.height * 2u);
-                    st.wrap_y = (int32_t)((uint32_t)st.wrap_y * 2u - (uint32_t)kTurbPerlinN);
-                }
-            }
-            const double v = tp.fractal ? __ddiv_rn(__dadd_rn(__dmul_rn(sum, 255.0), 255.0), 2.0) : __dmul_rn(sum, 255.0);
+        }
+        uint32_t px = 0;
+#pragma unroll
+        for (int ch = 0; ch < 4; ch++) {
+            const double m = __dmul_rn(sum[ch], 255.0);
+            const double v = tp.fractal ? __dmul_rn(__dadd_rn(m, 255.0), 0.5) : m;
             px |= sat_u8f(f32_bound(0.0f, __double2float_rn(v), 255.0f) + 0.5f) << (8 * ch);
         }
         out[idx] = tab_px(TAB_MUL, px);
