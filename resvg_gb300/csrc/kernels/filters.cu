@@ -1066,14 +1066,26 @@ __global__ void k_crop(uint32_t *img, int w, int h, int l, int t, int r, int b) 
 }
 // draw_pixmap(dx, dy, src) onto dst with a blend mode (highp, Nearest, opacity
 // 1): src is sw x sh, dst dw x dh; only the overlap is drawn
-__global__ void k_draw(const uint32_t *src, int sw, int sh, uint32_t *dst, int dw, int dh, int dx, int dy,
-                       uint32_t blend) {
-    size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)dw * dh) return;
-    int x = (int)(i % dw), y = (int)(i / dw);
-    int64_t sx = (int64_t)x - dx, sy = (int64_t)y - dy;
-    if (sx < 0 || sy < 0 || sx >= sw || sy >= sh) return;
-    dst[i] = dev::composite_pixel(src[(size_t)sy * sw + (size_t)sx], dst[i], 1.0f, blend);
+// draw_pixmap over the part of dst that src covers: w x h pixels from (x0, y0).
+// One row per block row, so that no pixel needs a division to find its place, and
+// four pixels per thread, loaded before the first is blended (12 us for 1920 x
+// 1080 with a 64-bit division per pixel, one pixel per thread).
+constexpr int kDrawPx = 4;
+__global__ void __launch_bounds__(256) k_draw(const uint32_t *src, size_t sw, uint32_t *dst, size_t dw, int w, int dx,
+                                              int dy, int x0, int y0, uint32_t blend) {
+    const int x = (int)(blockIdx.x * 256 * kDrawPx + threadIdx.x), y = y0 + (int)blockIdx.y;
+    const uint32_t *sp = src + (size_t)((int64_t)y - dy) * sw + (size_t)((int64_t)x0 - dx);
+    uint32_t *dp = dst + (size_t)y * dw + x0;
+    uint32_t a[kDrawPx], b[kDrawPx];
+#pragma unroll
+    for (int k = 0; k < kDrawPx; k++)
+        if (x + 256 * k < w) {
+            a[k] = sp[x + 256 * k];
+            b[k] = dp[x + 256 * k];
+        }
+#pragma unroll
+    for (int k = 0; k < kDrawPx; k++)
+        if (x + 256 * k < w) dp[x + 256 * k] = dev::composite_pixel(a[k], b[k], 1.0f, blend);
 }
 __global__ void k_fill(uint32_t *img, size_t n, uint32_t v) {
     auto f = [v](uint32_t) { return v; };
@@ -1089,9 +1101,14 @@ cudaError_t filter_crop(uint32_t *img, int w, int h, int l, int t, int r, int b,
 }
 cudaError_t filter_draw(const uint32_t *src, int sw, int sh, uint32_t *dst, int dw, int dh, int dx, int dy,
                         uint32_t blend, cudaStream_t s) {
-    size_t n = (size_t)dw * dh;
-    if (!n || sw <= 0 || sh <= 0) return cudaSuccess;
-    k_draw<<<nblk(n, 256), 256, 0, s>>>(src, sw, sh, dst, dw, dh, dx, dy, blend);
+    if (sw <= 0 || sh <= 0) return cudaSuccess;
+    const int64_t x0 = std::max<int64_t>(0, dx), x1 = std::min<int64_t>(dw, (int64_t)dx + sw);
+    const int64_t y0 = std::max<int64_t>(0, dy), y1 = std::min<int64_t>(dh, (int64_t)dy + sh);
+    if (x1 <= x0) return cudaSuccess;
+    // at most 65535 rows a launch
+    for (int64_t y = y0; y < y1; y += 65535)
+        k_draw<<<dim3(nblk((size_t)(x1 - x0), 256 * kDrawPx), (unsigned)std::min<int64_t>(65535, y1 - y)), 256, 0, s>>>(
+            src, (size_t)sw, dst, (size_t)dw, (int)(x1 - x0), dx, dy, (int)x0, (int)y, blend);
     return cudaGetLastError();
 }
 cudaError_t filter_fill(uint32_t *img, size_t n, uint32_t v, cudaStream_t s) {
@@ -1303,19 +1320,32 @@ __global__ void k_component_transfer(uint32_t *img, size_t n, Lut256 lut) {
 // flooded, colour-space converted shadow is a function of the blurred alpha
 // alone (a 256-entry table); it is drawn at (dx, dy) onto a transparent
 // image, then the input is drawn over it, both source-over.
-__global__ void k_drop_shadow(const uint32_t *in, const uint32_t *shadow, uint32_t *out, int w, int h, int dx,
-                              int dy, Lut256 lut) {
+// (one row per block row, four pixels per thread: see k_draw)
+__global__ void __launch_bounds__(256) k_drop_shadow(const uint32_t *in, const uint32_t *shadow, uint32_t *out, int w,
+                                                     int h, int dx, int dy, int y0, Lut256 lut) {
     __shared__ uint32_t s_lut[256];
-    for (int k = threadIdx.x; k < 256; k += blockDim.x) s_lut[k] = lut.v[k];
+    s_lut[threadIdx.x] = lut.v[threadIdx.x];
     __syncthreads();
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)w * h) return;
-    const int x = (int)(i % w), y = (int)(i / w);
-    const int64_t sx = (int64_t)x - dx, sy = (int64_t)y - dy;
-    uint32_t d = 0;
-    if (sx >= 0 && sy >= 0 && sx < w && sy < h)
-        d = dev::composite_pixel(s_lut[shadow[(size_t)sy * w + (size_t)sx] >> 24], 0u, 1.0f, RGPU_BLEND_SOURCE_OVER);
-    out[i] = dev::composite_pixel(in[i], d, 1.0f, RGPU_BLEND_SOURCE_OVER);
+    const int x = (int)(blockIdx.x * 256 * kDrawPx + threadIdx.x), y = y0 + (int)blockIdx.y;
+    const int64_t sy = (int64_t)y - dy;
+    const size_t row = (size_t)y * w;
+    uint32_t a[kDrawPx], c[kDrawPx];
+#pragma unroll
+    for (int k = 0; k < kDrawPx; k++) {
+        const int64_t px = x + 256 * k, sx = px - dx;
+        c[k] = 0;
+        if (px < w) {
+            a[k] = in[row + (size_t)px];
+            if (sx >= 0 && sy >= 0 && sx < w && sy < h) c[k] = shadow[(size_t)sy * w + (size_t)sx] | 1u;  // marked: inside
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kDrawPx; k++)
+        if (x + 256 * k < w) {
+            uint32_t d = 0;
+            if (c[k]) d = dev::composite_pixel(s_lut[c[k] >> 24], 0u, 1.0f, RGPU_BLEND_SOURCE_OVER);
+            out[row + (size_t)(x + 256 * k)] = dev::composite_pixel(a[k], d, 1.0f, RGPU_BLEND_SOURCE_OVER);
+        }
 }
 
 }  // namespace
@@ -1354,7 +1384,9 @@ cudaError_t filter_drop_shadow(const uint32_t *in, const uint32_t *shadow, uint3
         l.v[sa] = (uint32_t)g_host_tab[t][(pa << 8) | pr] | ((uint32_t)g_host_tab[t][(pa << 8) | pg] << 8) |
                   ((uint32_t)g_host_tab[t][(pa << 8) | pb] << 16) | (pa << 24);
     }
-    k_drop_shadow<<<nblk(n, 256), 256, 0, s>>>(in, shadow, out, w, h, dx, dy, l);
+    for (int y = 0; y < h; y += 65535)
+        k_drop_shadow<<<dim3(nblk((size_t)w, 256 * kDrawPx), (unsigned)std::min(65535, h - y)), 256, 0, s>>>(
+            in, shadow, out, w, h, dx, dy, y, l);
     return cudaGetLastError();
 }
 }  // namespace rgpu
