@@ -770,8 +770,7 @@ int enqueue_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, RasterTimer *t
         uint32_t tot = 0;
         CK(cudaMemcpyAsync(&tot, totals + 1, 4, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        // lists are placed by 32-bit bin offsets and slots
-        if ((uint64_t)tot + p.nbins >= 0xFFFFFFFFull) {
+        if (tot == 0xFFFFFFFFu) {  // where the scan's total saturates: bin offsets are 32-bit
             set_error("the submission's rows hold too many edges: render fewer scenes at a time");
             return RGPU_ERR_CAPACITY;
         }

@@ -518,6 +518,10 @@ k_raster(uint32_t max_row_w, const StreamRec *streams, const WorkItem *items, ui
         };
         int32_t depth = 0;
         const uint32_t row_slot = st.bin_off + wi.row * st.draw_cnt - st.draw_off;  // + draw: its slot
+        // the row's lists start here (offsets and slots each fit 32 bits, their sum may not)
+        const uint32_t slot0 = st.bin_off + wi.row * st.draw_cnt, off0 = __ldg(bin_offsets + slot0);
+        const uint32_t row_loc = off0 + slot0;
+        const uint32_t *row_events = events + 4ull * ((unsigned long long)off0 + slot0);
         bool stop = false, failed = false;
         for (uint32_t ci = 0, buf = 0; ci < ncmd && !stop; ci += kChunk, buf ^= 1u) {
             if (!wait_chunk(ws, copies & 1u, wait_limit)) {
@@ -542,9 +546,10 @@ k_raster(uint32_t max_row_w, const StreamRec *streams, const WorkItem *items, ui
                     n = h >> 20;
                     if (n == dev::kManyEvents) n = h & dev::kMaxEvents;
                     else if ((int32_t)(h >> 10 & 0x3FFu) > (x1 - 1) >> 5 || (int32_t)(h & 0x3FFu) < x0 >> 5) n = 0;
-                    if (n) loc = __ldg(bin_offsets + slot) + slot;
+                    if (n) loc = __ldg(bin_offsets + slot) + slot - row_loc;
                 }
             }
+            auto list_of = [&](int s) { return row_events + 4ull * __shfl_sync(0xffffffffu, loc, s); };
             uint32_t todo = __ballot_sync(0xffffffffu, my_op != kNone && (my_op != CMD_FILL || n != 0u));
             const uint32_t with_events = __ballot_sync(0xffffffffu, n != 0u);
             // copies what the first fill of `from` needs into slot `par`
@@ -555,7 +560,7 @@ k_raster(uint32_t max_row_w, const StreamRec *streams, const WorkItem *items, ui
                     FillSlot &f = ws.fill[par];
                     const Cmd &c = chunk[s];
                     const uint32_t g = __float_as_uint(c.f);  // the gradient, if any
-                    const uint32_t *list = events + 4ull * __shfl_sync(0xffffffffu, loc, s);
+                    const uint32_t *list = list_of(s);
                     if ((uint32_t)lane < __shfl_sync(0xffffffffu, n, s)) cp_async<4>(&f.events[lane], list + lane);
                     if (lane < 24) {
                         if (g != kNone) cp_async<16>(&f.rows[lane], reinterpret_cast<const uint4 *>(grads[g].iv) + lane);
@@ -579,7 +584,7 @@ k_raster(uint32_t max_row_w, const StreamRec *streams, const WorkItem *items, ui
                     const FillSlot &f = ws.fill[par];
                     uint32_t groups = 0;
                     if (cnt) {
-                        const uint32_t *list = events + 4ull * __shfl_sync(0xffffffffu, loc, cl);
+                        const uint32_t *list = list_of(cl);
                         par ^= 1u;
                         load_fill(todo);
                         cp_wait<1>();  // all but the copies just asked for
