@@ -191,13 +191,15 @@ __device__ __forceinline__ uint32_t path_nverts(const rgpu_soft_batch &B, uint32
 // composite is a chain over the paths but independent per pixel: a warp per few
 // groups of 32 pixels of a row.  Between them go, per (row, path), the areas (in
 // the adjoint later dL/dA), the colours under the path, and a mask of the
-// groups the path covers.  The scenes are taken in slices of bounded scratch.
+// groups the path covers.  The scenes, and the rows of a scene that is too large
+// by itself, are taken in slices of bounded scratch.
 // On 16 scenes of 64 paths on 256^2 pixels: areas 0.32 ms, composite 0.16 ms, its
 // reverse 0.72 ms, line gradients 0.32 ms.  (One CTA per row doing all of it in
 // turn, with a block barrier for every step of every path, took 1.10 ms forward
 // and 5.42 ms for the adjoint.)
 struct Slice {
-    uint32_t s0, scenes;  // scenes of the batch
+    uint32_t s0, scenes;  // scenes of the batch,
+    uint32_t row0, rows;  // these rows of each
     uint32_t ng;          // 32-pixel groups per row
     float *area;          // [scene, row][path][32 ng]
     float4 *under;        // adjoint: the colours under each path, likewise
@@ -289,13 +291,13 @@ __device__ __forceinline__ Fix fix40(float v) {
 __global__ void __launch_bounds__(32 * kRowWarps)
 k_area(rgpu_soft_batch B, Slice sl, const float2 *verts, uint32_t *overflow) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const uint32_t H = B.height, P = B.paths_per_scene;
+    const uint32_t H = sl.rows, P = B.paths_per_scene;
     const int W = (int)B.width, lane = threadIdx.x & 31;
     const RowMem rm = row_mem(smem, sl.ng);
     const uint32_t id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (id >= sl.scenes * P * H) return;
     // neighbouring warps: neighbouring rows of one path
-    const uint32_t row = id % H, sp = id / H, p = sp % P, sc = sp / P, j = (sl.s0 + sc) * P + p;
+    const uint32_t r = id % H, row = sl.row0 + r, sp = id / H, p = sp % P, sc = sp / P, j = (sl.s0 + sc) * P + p;
     const int E = 1 << rm.esh;
     for (int x = lane; x < 32 * E + 33; x += 32) rm.a[x] = rm.b[x] = 0;
     __syncwarp();
@@ -315,7 +317,7 @@ k_area(rgpu_soft_batch B, Slice sl, const float2 *verts, uint32_t *overflow) {
         if (xr < W) add(xr, fix40(c.z), prev);
     });
     if (lane == 0 && total >= (uint32_t)kMaxCross) atomicOr(overflow, 1u);
-    const size_t at = ((size_t)(sc * H + row) * P + p);
+    const size_t at = ((size_t)(sc * H + r) * P + p);
     uint32_t mask = 0;
     if (total) {
         // scan: each lane a run of E pixels
@@ -365,15 +367,17 @@ __device__ __forceinline__ void composite(float4 &C, float A, const PaintOut &po
 // the warp's row and groups: G neighbouring groups of one row
 template <int G>
 struct Strip {
-    uint32_t sc, row, g0;
+    uint32_t sc, row, g0;  // scene of the slice, row of the scene, first group
+    uint32_t r;            // row of the slice
     bool ok;
     __device__ __forceinline__ Strip(const rgpu_soft_batch &B, const Slice &sl) {
         const uint32_t per_row = (sl.ng + G - 1) / G;
-        const uint32_t id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), r = id / per_row;
+        const uint32_t id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+        r = id / per_row;
         g0 = (id - r * per_row) * G;
-        sc = r / B.height;
-        row = r - sc * B.height;
-        ok = r < sl.scenes * B.height;
+        sc = r / sl.rows;
+        row = sl.row0 + r - sc * sl.rows;
+        ok = r < sl.scenes * sl.rows;
     }
 };
 
@@ -387,7 +391,7 @@ __global__ void __launch_bounds__(128) k_composite(rgpu_soft_batch B, Slice sl, 
     float4 C[G];
 #pragma unroll
     for (int k = 0; k < G; k++) C[k] = make_float4(0.f, 0.f, 0.f, 0.f);
-    const size_t r = (size_t)st.sc * B.height + st.row;
+    const size_t r = st.r;
     for (uint32_t p0 = 0; p0 < P; p0 += 32) {
         // 32 paths' masks at a time; those without coverage here are skipped
         const uint32_t m = p0 + (uint32_t)lane < P ? (sl.mask[r * P + p0 + (uint32_t)lane] >> st.g0) & ((1u << G) - 1u) : 0u;
@@ -607,7 +611,7 @@ __global__ void __launch_bounds__(128) k_reverse(rgpu_soft_batch B, Slice sl, rg
     if (!st.ok) return;
     const int lane = threadIdx.x & 31, W = (int)B.width;
     const uint32_t P = B.paths_per_scene;
-    const size_t r = (size_t)st.sc * B.height + st.row, stride = 32 * (size_t)sl.ng;
+    const size_t r = st.r, stride = 32 * (size_t)sl.ng;
     const size_t first = r * P * stride + 32 * st.g0 + (uint32_t)lane;
     const float py = (float)st.row + 0.5f;
     float4 C[G], gC[G];
@@ -766,13 +770,13 @@ __device__ __forceinline__ float mean_right_d(float a, float b, float *da, float
 __global__ void __launch_bounds__(32 * kRowWarps)
 k_lines(rgpu_soft_batch B, Slice sl, const float2 *verts, float2 *vgrad) {
     extern __shared__ __align__(16) unsigned char smem[];
-    const uint32_t H = B.height, P = B.paths_per_scene;
+    const uint32_t H = sl.rows, P = B.paths_per_scene;
     const int W = (int)B.width, lane = threadIdx.x & 31;
     const RowMem rm = row_mem(smem, sl.ng);
     const uint32_t id = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (id >= sl.scenes * P * H) return;
-    const uint32_t row = id % H, sp = id / H, p = sp % P, sc = sp / P, j = (sl.s0 + sc) * P + p;
-    const size_t at = ((size_t)(sc * H + row) * P + p);
+    const uint32_t r = id % H, row = sl.row0 + r, sp = id / H, p = sp % P, sc = sp / P, j = (sl.s0 + sc) * P + p;
+    const size_t at = ((size_t)(sc * H + r) * P + p);
     const uint32_t mask = sl.mask[at];
     if (!mask) return;
     const int E = 1 << rm.esh;
@@ -886,20 +890,21 @@ int fail(cudaError_t e) {
 }
 
 // The scratch of a slice of scenes: areas and masks per (row, path), and for the
-// adjoint the colours under each path; at least one scene.  Slices that fit the
+// adjoint the colours under each path; at least one row of one scene.  Slices that fit the
 // L2 cache instead (96 MB, one scene of 64 paths on 256^2 pixels each) leave the
 // SMs short of warps: the four kernels took 3.25 ms against 1.84.
 constexpr size_t kSliceBytes = (size_t)1536 << 20;
 cudaError_t make_slice(const rgpu_soft_batch &b, bool adjoint, Slice *sl) {
     sl->ng = (b.width + 31) / 32;
-    const size_t rows = (size_t)b.height * b.paths_per_scene, px = rows * 32 * sl->ng;
-    const size_t per = px * (adjoint ? 20 : 4) + rows * 4;
-    sl->scenes = (uint32_t)std::min<size_t>(b.scenes, std::max<size_t>(1, kSliceBytes / per));
-    // warps are counted in 32 bits
-    sl->scenes = (uint32_t)std::min<size_t>(sl->scenes, std::max<size_t>(1, 0x7FFFFFFFull / rows));
-    cudaError_t e = g_area.ensure(sl->scenes * px * sizeof(float));
-    if (e == cudaSuccess && adjoint) e = g_col.ensure(sl->scenes * px * sizeof(float4));
-    if (e == cudaSuccess) e = g_mask.ensure(sl->scenes * rows * 4);
+    const size_t P = b.paths_per_scene, row_px = P * 32 * sl->ng;
+    // rows that fit; warps, one per (row, path) or group of a row, are counted in 32 bits
+    const size_t fit = std::min<size_t>(kSliceBytes / (row_px * (adjoint ? 20 : 4) + P * 4), 0x7FFFFFFFull / (P + sl->ng));
+    sl->rows = (uint32_t)std::min<size_t>(b.height, std::max<size_t>(1, fit));
+    sl->scenes = (uint32_t)std::min<size_t>(b.scenes, std::max<size_t>(1, fit / b.height));
+    const size_t rows = (size_t)sl->scenes * sl->rows;
+    cudaError_t e = g_area.ensure(rows * row_px * sizeof(float));
+    if (e == cudaSuccess && adjoint) e = g_col.ensure(rows * row_px * sizeof(float4));
+    if (e == cudaSuccess) e = g_mask.ensure(rows * P * 4);
     sl->area = (float *)g_area.p;
     sl->under = (float4 *)g_col.p;
     sl->mask = (uint32_t *)g_mask.p;
@@ -916,7 +921,7 @@ uint32_t blocks(uint64_t n, uint32_t per) { return (uint32_t)((n + per - 1) / pe
 // paths, would leave the SMs too little to do.  Reverse composite of 16 scenes of
 // 256^2 pixels: two 0.72 ms, four 0.77, eight 1.12.
 bool wide_strips(const rgpu_soft_batch &b, const Slice &sl) {
-    return sl.ng >= 2 && (uint64_t)sl.scenes * b.height * sl.ng >= 8192;
+    return sl.ng >= 2 && (uint64_t)sl.scenes * sl.rows * sl.ng >= 8192;
 }
 template <class F>
 void with_groups(bool wide, F f) {
@@ -926,16 +931,19 @@ void with_groups(bool wide, F f) {
 // f(slice) over the batch's scenes; launch errors are left for the caller's check
 template <class F>
 void each_slice(const rgpu_soft_batch &b, Slice sl, F f) {
-    const uint32_t most = sl.scenes;
-    for (uint32_t s0 = 0; s0 < b.scenes; s0 += most) {
-        sl.s0 = s0;
-        sl.scenes = std::min(most, b.scenes - s0);
-        f(sl);
-    }
+    const uint32_t most = sl.scenes, most_rows = sl.rows;
+    for (uint64_t s0 = 0; s0 < b.scenes; s0 += most)
+        for (uint64_t r0 = 0; r0 < b.height; r0 += most_rows) {
+            sl.s0 = (uint32_t)s0;
+            sl.scenes = (uint32_t)std::min<uint64_t>(most, b.scenes - s0);
+            sl.row0 = (uint32_t)r0;
+            sl.rows = (uint32_t)std::min<uint64_t>(most_rows, b.height - r0);
+            f(sl);
+        }
 }
 void launch_area(const rgpu_soft_batch &b, const Slice &sl, cudaStream_t s) {
     const uint32_t nw = row_warps(sl);
-    k_area<<<blocks((uint64_t)sl.scenes * b.paths_per_scene * b.height, nw), 32 * nw, nw * row_bytes(sl.ng), s>>>(
+    k_area<<<blocks((uint64_t)sl.scenes * b.paths_per_scene * sl.rows, nw), 32 * nw, nw * row_bytes(sl.ng), s>>>(
         b, sl, (const float2 *)g_verts.p, (uint32_t *)g_flags.p);
 }
 
@@ -982,7 +990,7 @@ extern "C" int rgpu_soft_forward(const rgpu_soft_batch *b, float *image, float *
         launch_area(*b, sl, s);
         with_groups(wide_strips(*b, sl), [&](auto G) {
             constexpr int kG = decltype(G)::value;
-            const uint64_t warps = (uint64_t)sl.scenes * b->height * ((sl.ng + kG - 1) / kG);
+            const uint64_t warps = (uint64_t)sl.scenes * sl.rows * ((sl.ng + kG - 1) / kG);
             k_composite<kG><<<blocks(warps, 4), 128, 0, s>>>(*b, sl, (float4 *)image);
         });
     });
@@ -1044,11 +1052,11 @@ extern "C" int rgpu_soft_backward(const rgpu_soft_batch *b, const float *image, 
         launch_area(*b, sl, s);
         with_groups(wide_strips(*b, sl), [&](auto G) {
             constexpr int kG = decltype(G)::value;
-            const uint64_t warps = (uint64_t)sl.scenes * b->height * ((sl.ng + kG - 1) / kG);
+            const uint64_t warps = (uint64_t)sl.scenes * sl.rows * ((sl.ng + kG - 1) / kG);
             k_reverse<kG><<<blocks(warps, 4), 128, 0, s>>>(*b, sl, *g, gI);
         });
         const uint32_t nw = row_warps(sl);
-        k_lines<<<blocks((uint64_t)sl.scenes * b->paths_per_scene * b->height, nw), 32 * nw, nw * row_bytes(sl.ng), s>>>(
+        k_lines<<<blocks((uint64_t)sl.scenes * b->paths_per_scene * sl.rows, nw), 32 * nw, nw * row_bytes(sl.ng), s>>>(
             *b, sl, (const float2 *)g_verts.p, (float2 *)g_vgrad.p);
     });
     dim3 ug(1, npaths);

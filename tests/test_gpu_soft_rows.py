@@ -45,3 +45,9 @@ def test_rows_match_fp64(gpu, oracle_mod, scenes, w, h, paths):
     terms = np.concatenate([(grads[k].double().cpu().numpy() * v[k]).ravel() for k in KEYS])
     _, ref = oracle_mod.soft_dloss(a, target.cpu().numpy(), v)
     assert abs(terms.sum() - ref) <= 1e-3 * np.abs(terms).sum()
+
+
+def test_rows_of_a_large_scene(gpu, oracle_mod):
+    # more scratch than a slice holds: the rows of one scene in slices (280 and 10
+    # forward, 56 rows at a time in the adjoint)
+    test_rows_match_fp64(gpu, oracle_mod, 1, 1024, 290, 1400)
