@@ -412,7 +412,7 @@ def run_batched(args, rank, world):
     torch.cuda.set_stream(stream)
     sh = stream.cuda_stream
     # autotune the raster decomposition on a stratified sample of the scenes:
-    # band rows per (canvas-width, draw-count) bucket, then pixels per thread
+    # band rows per (canvas-width, draw-count) bucket (kept, without effect), then pixels per thread
     samp = list(range(0, n, max(1, n // 256)))
     t0 = time.perf_counter()
     table, best_px, tune_ms = BT.autotune_table([trees[i] for i in samp], [ws[i] for i in samp],
@@ -526,7 +526,7 @@ def run_batched(args, rank, world):
         "batched_vs_plain": value / plain_value / max(1, world),
         "raster_ms": rms,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
-                     "peak_kind": peak_kind, "traffic": profiled_traffic("config3"), "kernel": "k_raster (band VM)",
+                     "peak_kind": peak_kind, "traffic": profiled_traffic("config3"), "kernel": "k_raster",
                      "algorithmic_bytes": alg_bytes, "issue_roof": profiled_issue("config3")},
         "e2e": {"value": n_total * 1e3 / e2e_ms, "unit": "scenes/s", "ms_per_step": e2e_ms,
                 "h2d_bytes_per_step": int(st["h2d_bytes"]), "d2h_bytes_per_step": int(total),
@@ -770,7 +770,7 @@ def run_plain(args, rank, world):
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                      "frac": achieved / peak, "peak_kind": peak_kind,
                      "traffic": profiled_traffic("config%d" % args.config),
-                     "kernel": "k_raster (band VM)", "algorithmic_bytes": alg_bytes,
+                     "kernel": "k_raster", "algorithmic_bytes": alg_bytes,
                      "issue_roof": profiled_issue("config%d" % args.config)},
         "e2e": {"value": 1e3 / e2e_ms, "unit": "scenes/s", "ms_per_step": e2e_ms,
                 "h2d_bytes_per_step": int(st["h2d_bytes"]), "d2h_bytes_per_step": int(st["d2h_bytes"])},

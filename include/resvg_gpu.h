@@ -124,7 +124,7 @@ int rgpu_render_batch(const resvg_render_tree *const *trees, const resvg_transfo
  * The first render sizes the edge/bin buffers (two stream synchronisations);
  * later renders are asynchronous and replay a captured CUDA graph.  The
  * device pixmaps given at prepare time are the render targets.  The batched
- * form (many trees) uses one persistent raster kernel over all scenes' bands. */
+ * form (many trees) uses one persistent raster kernel over all scenes' rows. */
 typedef struct rgpu_scene rgpu_scene;
 int rgpu_scene_prepare(const resvg_render_tree *const *trees, const resvg_transform *transforms, uint32_t count,
                        const uint32_t *widths, const uint32_t *heights, uint8_t *const *device_pixmaps,

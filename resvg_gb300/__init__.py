@@ -378,9 +378,9 @@ def stroke_paths(paths, on_device: bool = True):
 
 
 def set_tuning_table(entries) -> None:
-    """Band rows per (max stream width, max stream draws) bucket, used for
-    streams whose band rows the tuning leaves automatic: entries are
-    (max_width, max_draws, band_rows) tuples, first match wins."""
+    """Band rows per (max stream width, max stream draws) bucket, kept
+    and returned as set (work items are single rows, so they choose nothing):
+    entries are (max_width, max_draws, band_rows) tuples."""
     L = lib()
     L.rgpu_set_tuning_table.restype = C.c_int
     L.rgpu_set_tuning_table.argtypes = [C.POINTER(_abi.TuningEntry), C.c_uint32]

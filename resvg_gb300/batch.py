@@ -13,8 +13,9 @@ import heapq
 
 import numpy as np
 
-# (band rows, pixels per thread) the autotuner searches; band rows 0 = chosen
-# per stream from its width.
+# (band rows, pixels per thread) the autotuner searches.  Work items are single
+# rows, so band rows make no difference; pixels per thread set the width of a row
+# piece (32 times as many pixels).
 TUNING_CANDIDATES = [(0, 8), (0, 16), (1, 4), (2, 4), (4, 4), (2, 8), (4, 8), (8, 8), (4, 16), (8, 16)]
 
 # Buckets of the tuning table: stream width (canvas side) and draws (fills and

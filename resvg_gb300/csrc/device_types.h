@@ -7,9 +7,9 @@
 //                 target layer, the layer size (the tiny-skia clip rect) and paint;
 //   * PaintRec  — the resolved paint in the form the raster pipeline consumes;
 //   * LayerRec  — isolated-group layers / clip and mask pixmaps (integer rects);
-//   * Cmd       — the command stream the band VM executes in order.
+//   * Cmd       — the command stream the raster kernel executes in order.
 // Geometry (verbs, f32 points) is uploaded as-is; the device transforms points,
-// builds fixed-point edges, bins them into row bands and rasterises.
+// builds fixed-point edges, bins them by row and rasterises.
 #pragma once
 #include <stdint.h>
 #include <stddef.h>
@@ -171,7 +171,7 @@ struct WorkItem {
     int32_t x0, x1;
 };
 
-// One stream = one target surface rendered by the band VM.
+// One stream = one target surface rendered by the raster kernel.
 struct StreamRec {
     uint32_t cmd_off, cmd_cnt;
     uint32_t draw_off, draw_cnt;   // draws referenced by this stream

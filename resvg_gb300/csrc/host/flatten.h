@@ -1,7 +1,7 @@
 // Host flattener: walks a render tree the way resvg's renderer does
 // (crates/resvg/src/render.rs:10-142, path.rs:6-177, clip.rs:6-98,
 // mask.rs:6-46) and emits device records (draws, paints, gradients, layers)
-// and the band VM's command streams instead of rasterising.
+// and the raster kernel's command streams instead of rasterising.
 //
 // A group with filters (render.rs:113-117) splits the work: its content is
 // flattened into a stream of its own that renders into an internal surface at

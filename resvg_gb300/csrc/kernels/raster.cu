@@ -1,4 +1,4 @@
-// The band VM: one persistent kernel renders every work item (a row of a stream,
+// The raster kernel: one persistent kernel renders every work item (a row of a stream,
 // or a piece of it) by executing the stream's command list, one warp per item.
 //
 // Per draw, the warp adds the row's coverage events (events.cuh) to a difference
