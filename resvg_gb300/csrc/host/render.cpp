@@ -727,6 +727,9 @@ int upload_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, HostBuf *stagin
     return RGPU_OK;
 }
 
+// kernels of a render of a sized plan (without filters and further raster levels)
+uint32_t plan_launches(const Plan &p) { return 8 + scan_launches(p.nsegs + 1) + scan_launches(p.nbins + 1); }
+
 // Enqueues the device pipeline.  Without known sizes it synchronises twice to
 // read the edge and bin totals; with known sizes (a prepared scene rendered
 // before) it is fully asynchronous and capturable into a CUDA graph.
@@ -830,7 +833,7 @@ int enqueue_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, RasterTimer *t
     }
     g_stats.draws += ndraws;
     g_stats.work_items += p.items.size();
-    g_stats.kernel_launches += 14;
+    g_stats.kernel_launches += plan_launches(p);
     return RGPU_OK;
 }
 
@@ -1290,7 +1293,7 @@ int rgpu_scene_info(const rgpu_scene *sc, rgpu_scene_stats *st) {
     st->work_items = p.items.size();
     st->grid = p.grid;
     st->pixels_per_thread = p.row_w / 32;
-    st->kernel_launches = 14;
+    st->kernel_launches = plan_launches(sc->plan);
     uint64_t px = 0;
     for (auto &s : p.sb.streams) px += (uint64_t)s.out_w * s.out_h;
     st->output_pixels = px;

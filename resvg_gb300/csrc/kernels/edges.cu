@@ -380,6 +380,45 @@ __global__ void k_scan_down(const uint32_t *in, uint64_t n, const uint32_t *bloc
     }
 }
 
+// The whole scan in one block, for counts that one block holds in registers: the
+// three launches above are about 2.8 us each however little they do.  Sums are
+// 64-bit up to the total; offsets past a total that does not fit are not read.
+constexpr int SCAN_ONE_T = 1024;
+constexpr int SCAN_ONE_PER = 16;
+__global__ void __launch_bounds__(SCAN_ONE_T)
+k_scan_one(const uint32_t *in, uint32_t n, uint32_t per, uint32_t *out, uint32_t *total_out) {
+    __shared__ unsigned long long warp_sums[32];
+    const uint32_t lane = threadIdx.x & 31u, wid = threadIdx.x >> 5, base = threadIdx.x * per;
+    uint32_t v[SCAN_ONE_PER];
+    unsigned long long sum = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < (uint32_t)SCAN_ONE_PER; k++) {
+        v[k] = k < per && base + k < n ? in[base + k] : 0u;
+        sum += v[k];
+    }
+    unsigned long long x = sum;
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned long long y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= (uint32_t)o) x += y;
+    }
+    if (lane == 31u) warp_sums[wid] = x;
+    __syncthreads();
+    const unsigned long long w = warp_sums[lane];
+    unsigned long long before = lane < wid ? w : 0ull, all = w;
+    for (int o = 16; o; o >>= 1) {
+        before += __shfl_xor_sync(0xffffffffu, before, o);
+        all += __shfl_xor_sync(0xffffffffu, all, o);
+    }
+    unsigned long long at = before + x - sum;
+#pragma unroll
+    for (uint32_t k = 0; k < (uint32_t)SCAN_ONE_PER; k++) {
+        if (k < per && base + k < n) out[base + k] = (uint32_t)at;
+        at += v[k];
+    }
+    // a total that does not fit is reported as 2^32 - 1
+    if (threadIdx.x == 0) *total_out = (uint32_t)min(all, 0xFFFFFFFFull);
+}
+
 inline uint32_t blocks_for(uint64_t n, uint32_t t) { return (uint32_t)((n + t - 1) / t); }
 
 }  // namespace
@@ -424,11 +463,16 @@ cudaError_t launch_bin(bool scatter, const EdgeRec *edges, const uint32_t *edge_
                                                               bin_offsets, bin_cap, err, bins);
     return cudaGetLastError();
 }
+uint32_t scan_launches(uint64_t n) { return n <= (uint64_t)SCAN_ONE_T * SCAN_ONE_PER ? 1u : 3u; }
 size_t scan_scratch_words(uint64_t n) { return (size_t)blocks_for(n ? n : 1, SCAN_TILE) + 1; }
 // out[i] = sum(in[0..i)), *total = sum(in); `scratch` holds scan_scratch_words(n) words.
 cudaError_t launch_exclusive_scan(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *scratch, uint32_t *total,
                                   cudaStream_t s) {
     if (n == 0) return cudaMemsetAsync(total, 0, 4, s);
+    if (scan_launches(n) == 1) {
+        k_scan_one<<<1, SCAN_ONE_T, 0, s>>>(in, (uint32_t)n, blocks_for(n, SCAN_ONE_T), out, total);
+        return cudaGetLastError();
+    }
     uint32_t nb = blocks_for(n, SCAN_TILE);
     k_scan_reduce<<<nb, SCAN_T, 0, s>>>(in, n, scratch);
     k_scan_blocks<<<1, SCAN_T, 0, s>>>(scratch, nb, total);

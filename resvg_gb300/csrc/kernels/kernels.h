@@ -50,6 +50,7 @@ cudaError_t launch_bin(bool scatter, const EdgeRec *edges, const uint32_t *edge_
                        const DrawRec *draws, const StreamRec *streams, uint32_t *bin_counts,
                        const uint32_t *bin_offsets, uint32_t bin_cap, uint32_t *err, uint32_t *bins, cudaStream_t s);
 size_t scan_scratch_words(uint64_t n);
+uint32_t scan_launches(uint64_t n);  // kernels of a scan of n > 0 words
 cudaError_t launch_exclusive_scan(const uint32_t *in, uint32_t *out, uint64_t n, uint32_t *scratch, uint32_t *total,
                                   cudaStream_t s);
 
