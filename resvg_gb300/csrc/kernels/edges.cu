@@ -380,11 +380,14 @@ __global__ void k_scan_down(const uint32_t *in, uint64_t n, const uint32_t *bloc
     }
 }
 
-// The whole scan in one block, for counts that one block holds in registers: the
-// three launches above are about 2.8 us each however little they do.  Sums are
-// 64-bit up to the total; offsets past a total that does not fit are not read.
+// The whole scan in one block, bound by launch and load latency.  The three
+// launches above take 8.3 us and the gaps between them however little they do;
+// this one 4.0 us for 1,001 words, 4.7 for 4,096.  Threads read neighbouring runs,
+// so longer runs cost more transactions (16,381 words by 16 each: 15.1 us), and
+// the line is at 4 words per thread.  Sums are 64-bit up to the total; offsets past
+// a total that does not fit are not read.
 constexpr int SCAN_ONE_T = 1024;
-constexpr int SCAN_ONE_PER = 16;
+constexpr int SCAN_ONE_PER = 4;
 __global__ void __launch_bounds__(SCAN_ONE_T)
 k_scan_one(const uint32_t *in, uint32_t n, uint32_t per, uint32_t *out, uint32_t *total_out) {
     __shared__ unsigned long long warp_sums[32];

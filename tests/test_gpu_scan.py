@@ -1,4 +1,4 @@
-"""Offsets by the scan in one block (up to 16,384 words) and by three launches
+"""Offsets by the scan in one block (up to 4,096 words) and by three launches
 beyond: canvases whose (row, draw) slots end at either side of the limit and of
 one word per thread, against the oracle.  Pixels are integers computed by integer
 rules: the tolerance is 0 differing pixels.
@@ -13,7 +13,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("draws", [1, 3])
-@pytest.mark.parametrize("slots", [1, 1022, 1023, 1024, 8191, 16382, 16383, 16384, 16400, 30000])
+@pytest.mark.parametrize("slots", [1, 1022, 1023, 1024, 4094, 4095, 4096, 8191, 16382, 16383, 16384, 16400, 30000])
 def test_slots_around_the_limits(gpu, oracle_mod, slots, draws):
     w, h = 6, max(1, slots // draws)
     t = R.Tree(w, h)
