@@ -221,7 +221,9 @@ __device__ __forceinline__ void shade_groups(uint32_t mask, int bits_sh, const u
         mask &= mask - 1u;
     };
     uint32_t cv[2], d[2];
-    if (kind == 0) {
+    // a clear of an aliased path is a source of its memset colour, whatever the
+    // paint (its coverage is 0 or 255 only)
+    if (kind == 0 || (flags & PAINT_MEMSET)) {
         uint32_t rb = __byte_perm(p1.x, p1.y, 0x5410), ga = __byte_perm(p1.x, p1.y, 0x7632);
         if (flags & PAINT_MEMSET) {  // the colour where the pixel is fully covered (the same, or a clear)
             rb = dev::pair_rb(p2.z);
