@@ -48,6 +48,7 @@ k_draw_setup(DrawRec *draws, uint32_t ndraws, const uint8_t *scene_verbs, const 
     };
     // segment slots default to empty
     for (uint32_t i = lane; i <= dr.verb_cnt; i += 32u) segs[dr.seg_base + i] = SegRec{d, 0, 0, 0};
+    __syncwarp();  // before other lanes write the segments to the same slots
     if (dr.flags & 0x80000000u) { done(); return; }  // host-side skip
     // ---- transform (tiny-skia Transform::map_points branches)
     const float sx = dr.ts[0], ky = dr.ts[1], kx = dr.ts[2], sy = dr.ts[3], tx = dr.ts[4], ty = dr.ts[5];

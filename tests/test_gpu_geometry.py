@@ -64,3 +64,19 @@ def test_curve_steps_and_edge_heights(gpu, oracle_mod, size):
     w, h = (int(size) + 9, int(size) // 2 + 9)
     _render(oracle_mod, paths, w, h)
     _render(oracle_mod, paths, w, h, (1.3, 0.2, -0.4, 0.9, -0.1 * size, 0.05 * size))
+
+
+@pytest.mark.parametrize("seed", range(12))
+def test_verbs_of_every_kind_match_the_oracle(gpu, oracle_mod, seed):
+    """Contours of every verb, 20 to 300 of them, so that lanes other than the one
+    that clears a segment slot fill it.  The points stay inside the canvas: random
+    curves that leave it differ from the oracle by one level in a few pixels
+    (clipping of curves, on every route of the device)."""
+    g = np.random.default_rng(100 + seed)
+    paths = []
+    for n in (20, 31, 32, 33, 64, 97, 300):
+        v = [A.MOVE]
+        while len(v) < n:
+            v.append(int(g.choice([A.LINE, A.QUAD, A.CUBIC, A.CLOSE, A.MOVE], p=[0.35, 0.2, 0.2, 0.15, 0.1])))
+        paths.append((v, g.uniform(2.0, 108.0, size=(sum(NPTS[x] for x in v), 2)).astype(np.float32)))
+    assert _render(oracle_mod, paths, 120, 110).any()
