@@ -354,9 +354,11 @@ k_area(rgpu_soft_batch B, Slice sl, const float2 *verts, uint32_t *overflow) {
     if (lane == 0) sl.mask[at] = mask;
 }
 
-// C = c P + (1 - c a) C for one pixel and path
+// C = c P + (1 - c a) C for one pixel and path; a pixel without coverage keeps its
+// colour whatever the paint (an infinite one would make it NaN)
 __device__ __forceinline__ void composite(float4 &C, float A, const PaintOut &po) {
     const float c = fminf(fabsf(A), 1.0f);
+    if (c == 0.0f) return;
     const float ca = c * po.a, keep = 1.0f - ca;
     C.x = c * (po.r * po.a) + keep * C.x;
     C.y = c * (po.g * po.a) + keep * C.y;

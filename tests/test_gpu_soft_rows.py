@@ -51,3 +51,26 @@ def test_rows_of_a_large_scene(gpu, oracle_mod):
     # more scratch than a slice holds: the rows of one scene in slices (280 and 10
     # forward, 56 rows at a time in the adjoint)
     test_rows_match_fp64(gpu, oracle_mod, 1, 1024, 290, 1400)
+
+
+@pytest.mark.parametrize("bad", [np.inf, -np.inf, np.nan])
+@pytest.mark.parametrize("gradient", [0, 1])
+def test_non_finite_paint_stays_in_its_coverage(gpu, bad, gradient):
+    """A path with an infinite or NaN colour spoils the pixels it covers and no
+    others: those keep the colours of a scene where it is transparent."""
+    w, h = 70, 16
+    a = soft.make_scenes(seed=5, scenes=1, size=w, paths=3, min_segs=2, max_segs=3)
+    a["width"], a["height"] = w, h
+    a["paint_kind"][:] = (0, gradient, 0)
+    off = a["seg_offset"].astype(int)
+    a["points"] = a["points"].astype(np.float32)
+    a["points"][:, 1] *= h / w
+    lo, hi = 3 * off[1], 3 * off[2]
+    a["points"][lo:hi, 0] = 33.0 + (a["points"][lo:hi, 0] % 9.0)  # columns 33 .. 42 of a 32-pixel group
+    b = {k: np.copy(v) if isinstance(v, np.ndarray) else v for k, v in a.items()}
+    a["colors"][1], a["stop_colors"][1] = bad, bad
+    b["colors"][1], b["stop_colors"][1] = 0.0, 0.0
+    img, ref = (soft.forward(soft.Scenes(x))[0].cpu().numpy() for x in (a, b))
+    for part in (slice(0, 33), slice(43, w)):
+        assert np.isfinite(img[:, :, part]).all() and np.array_equal(img[:, :, part], ref[:, :, part])
+    assert not np.isfinite(img[:, :, 33:43]).all()  # the covered ones are spoilt
