@@ -185,9 +185,13 @@ int rgpu_set_wait_limit(uint32_t rounds);
  * their first commands, so that bounded wait must run out (no GPU fault is made);
  * rgpu_test_fail_allocations(n) makes the library's next n device or pinned
  * host allocations fail as if memory were exhausted (RGPU_ERR_OUT_OF_MEMORY,
- * the pixmap untouched). */
+ * the pixmap untouched);
+ * rgpu_test_scan runs the device's exclusive prefix sum over `count` host words
+ * (`offsets` and `total` are host words too; a total of 2^32 - 1 or more is
+ * reported as 2^32 - 1, and the offsets are then unspecified). */
 int rgpu_test_withhold_window(int enabled);
 int rgpu_test_fail_allocations(uint32_t count);
+int rgpu_test_scan(const uint32_t *counts, uint32_t count, uint32_t *offsets, uint32_t *total);
 /* rgpu_render_batch cuts a batch into chunks of about equal estimated cost
  * (pixels x paths) and flattens and uploads chunk k + 1 on the host while the
  * device renders chunk k.  `chunks` = 0: automatic (8 chunks for batches of

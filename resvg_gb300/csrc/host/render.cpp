@@ -1433,6 +1433,28 @@ int rgpu_test_fail_allocations(uint32_t count) {
     return RGPU_OK;
 }
 
+int rgpu_test_scan(const uint32_t *counts, uint32_t count, uint32_t *offsets, uint32_t *total) {
+    g_last_error.clear();
+    if (!counts || !count || !offsets || !total) { set_error("invalid arguments"); return RGPU_ERR_INVALID_ARG; }
+    Context &c = ctx();
+    std::lock_guard<std::mutex> lock(c.mu);
+    int r = ensure_device(c);
+    if (r) return r;
+    const size_t bytes = (size_t)count * 4;
+    Buffers &b = c.buf;
+    CK(b.bin_counts.ensure(bytes));
+    CK(b.bin_offsets.ensure(bytes));
+    CK(b.scan_scratch.ensure(scan_scratch_words(count) * 4));
+    CK(b.totals.ensure(64));
+    CK(cudaMemcpyAsync(b.bin_counts.p, counts, bytes, cudaMemcpyHostToDevice, c.stream));
+    CK(launch_exclusive_scan(b.bin_counts.as<uint32_t>(), b.bin_offsets.as<uint32_t>(), count,
+                             b.scan_scratch.as<uint32_t>(), b.totals.as<uint32_t>(), c.stream));
+    CK(cudaMemcpyAsync(offsets, b.bin_offsets.p, bytes, cudaMemcpyDeviceToHost, c.stream));
+    CK(cudaMemcpyAsync(total, b.totals.p, 4, cudaMemcpyDeviceToHost, c.stream));
+    CK(cudaStreamSynchronize(c.stream));
+    return RGPU_OK;
+}
+
 int rgpu_set_batch_chunks(uint32_t chunks) {
     Context &c = ctx();
     std::lock_guard<std::mutex> lock(c.mu);

@@ -312,55 +312,59 @@ constexpr int SCAN_T = 256;
 constexpr int SCAN_PER = 4;
 constexpr int SCAN_TILE = SCAN_T * SCAN_PER;
 
-__device__ __forceinline__ uint32_t block_exclusive(uint32_t v, uint32_t *sh, uint32_t *total) {
+template <class T>
+__device__ __forceinline__ T block_exclusive(T v, T *sh, T *total) {
     int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t x = v;
+    T x = v;
     for (int o = 1; o < 32; o <<= 1) {
-        uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        T y = __shfl_up_sync(0xffffffffu, x, o);
         if (lane >= o) x += y;
     }
     if (lane == 31) sh[wid] = x;
     __syncthreads();
     if (wid == 0) {
-        uint32_t w = lane < (SCAN_T / 32) ? sh[lane] : 0;
+        T w = lane < (SCAN_T / 32) ? sh[lane] : 0;
         for (int o = 1; o < 32; o <<= 1) {
-            uint32_t y = __shfl_up_sync(0xffffffffu, w, o);
+            T y = __shfl_up_sync(0xffffffffu, w, o);
             if (lane >= o) w += y;
         }
         if (lane < (SCAN_T / 32)) sh[lane] = w;
     }
     __syncthreads();
-    uint32_t warp_prefix = wid ? sh[wid - 1] : 0;
+    T warp_prefix = wid ? sh[wid - 1] : 0;
     *total = sh[SCAN_T / 32 - 1];
     __syncthreads();
     return warp_prefix + x - v;
 }
 
+// Sums that do not fit 32 bits are kept as 2^32 - 1, a tile's as well as the
+// total, so that the caller sees a total that does not fit (the offsets are not
+// used then); 64-bit sums in between.
+__device__ __forceinline__ uint32_t sat_u32(unsigned long long v) { return (uint32_t)min(v, 0xFFFFFFFFull); }
+
 __global__ void k_scan_reduce(const uint32_t *in, uint64_t n, uint32_t *block_sums) {
-    __shared__ uint32_t sh[32];
+    __shared__ unsigned long long sh[32];
     uint64_t base = (uint64_t)blockIdx.x * SCAN_TILE;
-    uint32_t s = 0;
+    unsigned long long s = 0;
     for (int k = 0; k < SCAN_PER; k++) {
         uint64_t i = base + (uint64_t)threadIdx.x * SCAN_PER + k;
         if (i < n) s += in[i];
     }
-    uint32_t total;
+    unsigned long long total;
     block_exclusive(s, sh, &total);
-    if (threadIdx.x == 0) block_sums[blockIdx.x] = total;
+    if (threadIdx.x == 0) block_sums[blockIdx.x] = sat_u32(total);
 }
 __global__ void k_scan_blocks(uint32_t *block_sums, uint32_t nblocks, uint32_t *total_out) {
-    __shared__ uint32_t sh[32];
-    uint64_t carry = 0;
+    __shared__ unsigned long long sh[32];
+    unsigned long long carry = 0;
     for (uint32_t base = 0; base < nblocks; base += SCAN_T) {
         uint32_t i = base + threadIdx.x;
-        uint32_t v = i < nblocks ? block_sums[i] : 0;
-        uint32_t tot;
-        uint32_t ex = block_exclusive(v, sh, &tot);
-        if (i < nblocks) block_sums[i] = (uint32_t)carry + ex;
+        unsigned long long v = i < nblocks ? block_sums[i] : 0, tot;
+        unsigned long long ex = block_exclusive(v, sh, &tot);
+        if (i < nblocks) block_sums[i] = (uint32_t)(carry + ex);
         carry += tot;
     }
-    // a total that does not fit is reported as 2^32 - 1
-    if (threadIdx.x == 0) *total_out = (uint32_t)min(carry, (uint64_t)0xFFFFFFFFu);
+    if (threadIdx.x == 0) *total_out = sat_u32(carry);
 }
 __global__ void k_scan_down(const uint32_t *in, uint64_t n, const uint32_t *block_sums, uint32_t *out) {
     __shared__ uint32_t sh[32];
@@ -419,8 +423,7 @@ k_scan_one(const uint32_t *in, uint32_t n, uint32_t per, uint32_t *out, uint32_t
         if (k < per && base + k < n) out[base + k] = (uint32_t)at;
         at += v[k];
     }
-    // a total that does not fit is reported as 2^32 - 1
-    if (threadIdx.x == 0) *total_out = (uint32_t)min(all, 0xFFFFFFFFull);
+    if (threadIdx.x == 0) *total_out = sat_u32(all);
 }
 
 inline uint32_t blocks_for(uint64_t n, uint32_t t) { return (uint32_t)((n + t - 1) / t); }

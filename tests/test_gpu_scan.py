@@ -3,6 +3,9 @@ beyond: canvases whose (row, draw) slots end at either side of the limit and of
 one word per thread, against the oracle.  Pixels are integers computed by integer
 rules: the tolerance is 0 differing pixels.
 """
+import ctypes as C
+
+import numpy as np
 import pytest
 
 import resvg_gb300 as R
@@ -27,3 +30,28 @@ def test_slots_around_the_limits(gpu, oracle_mod, slots, draws):
     got = R.render(t, (1, 0, 0, 1, 0, 0), w, h)
     assert diff_stats(got, oracle_mod.render(t.view(), (1, 0, 0, 1, 0, 0), w, h)) == (0, 0)
     assert got.any()
+
+
+@pytest.mark.parametrize("n", [1, 5, 1000, 1024, 4096, 4097, 5000, 262144, 300000])
+@pytest.mark.parametrize("total", [0, 1, 0xFFFFFFFE, 0xFFFFFFFF, 1 << 32, (1 << 32) + 5, 3 << 32, 1 << 40])
+def test_totals_that_do_not_fit(gpu, n, total):
+    """Counts whose sum passes 2^32 within one tile, within the 256 tiles summed at
+    a time, or over all of them: never a wrapped total, which would size the lists
+    too small."""
+    L = R.lib()
+    L.rgpu_test_scan.restype = C.c_int
+    L.rgpu_test_scan.argtypes = [C.c_void_p, C.c_uint32, C.c_void_p, C.POINTER(C.c_uint32)]
+    for heavy in {1, min(n, 3), min(n, 1024), n}:  # the counts the total is spread over
+        if total // heavy >= 1 << 32:
+            continue
+        counts = np.zeros(n, np.uint64)
+        at = np.linspace(0, n - 1, heavy).astype(np.int64)
+        counts[at] = total // heavy
+        counts[at[-1]] += total - int(counts.sum())
+        if counts.max() >= 1 << 32:
+            continue
+        c32, out, tot = counts.astype(np.uint32), np.empty(n, np.uint32), C.c_uint32(7)
+        assert L.rgpu_test_scan(c32.ctypes.data, n, out.ctypes.data, C.byref(tot)) == 0
+        assert tot.value == min(total, 0xFFFFFFFF)
+        if total < 0xFFFFFFFF:
+            assert np.array_equal(out, (np.cumsum(counts) - counts).astype(np.uint32))
