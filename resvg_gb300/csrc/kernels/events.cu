@@ -24,24 +24,32 @@ namespace {
 using dev::event_diffs;
 
 constexpr int kWarps = 8;
-constexpr int kCol = 32;         // events of a lane (one more than the crossings it sorts)
+constexpr int kCol = 32;         // events of a lane
+constexpr int kMaxSort = kCol - 2;  // crossings it sorts: the row's start and end may add an event each
 constexpr int kColStride = 33;   // words between a column's entries
 constexpr uint32_t kOver = 0xFFFFFFFFu;
 
 // A crossing's sort key: the x of an edge on the sub-scanline relative to the
-// row's first pixel, clamped to the row's pixels (16.16 sub-columns, below 2^31:
-// anti-aliased rows end below pixel 8192, aliased ones below 32768), and the
-// winding in the lowest bit (-1 first among equal x, as the reference's sort has
-// it; crossings of equal x and winding commute).  Where clamping merges
-// crossings left (right) of the row, only the winding at the row's first pixel
-// matters (nothing does), so their order is free.
-__device__ __forceinline__ bool crossing_key(const int4 &e, int32_t y, int32_t base, uint32_t xmax, uint32_t *key) {
+// row's first pixel (16.16 sub-columns, below 2^31: anti-aliased rows end below
+// pixel 8192, aliased ones below 32768), and the winding in the lowest bit (-1
+// first among equal x, as the reference's sort has it; crossings of equal x and
+// winding commute).  Only crossings inside the row have one: of those left of it
+// the sum of the windings matters alone, `before`, and of those right of it
+// nothing.  (A view into a drawing has many of both: its clipped contours run
+// along the clip's sides.)
+__device__ __forceinline__ bool crossing_key(const int4 &e, int32_t y, int32_t base, uint32_t xmax, uint32_t *key,
+                                             int32_t *before) {
     const int32_t dy = y - e.z;
     if ((uint32_t)dy > (uint32_t)(e.w >> 8)) return false;
     const int32_t X = (int32_t)((uint32_t)e.x + (uint32_t)dy * (uint32_t)e.y);
-    const uint32_t d = X > base ? min((uint32_t)X - (uint32_t)base, xmax) : 0u;
-    *key = (d << 1) | ((e.w & 0x80) ? 0u : 1u);
-    return true;
+    const uint32_t up = (e.w & 0x80) ? 0u : 1u;
+    if (X <= base) {
+        *before += (int32_t)(up << 1) - 1;
+        return false;
+    }
+    const uint32_t d = (uint32_t)X - (uint32_t)base;
+    *key = (d << 1) | up;
+    return d < xmax;
 }
 // the key's x rounded to a sub-column: ((key >> 1) + 0x8000) >> 16
 __device__ __forceinline__ uint32_t key_sub(uint32_t key) { return (key + 0x10000u) >> 17; }
@@ -72,68 +80,84 @@ struct RowScan {
     int32_t fill_mask;     // 1 even-odd, -1 non-zero
 };
 
-// A sub-scanline with more crossings than a column holds, by a whole warp:
-// each lane takes an edge and sums the windings of the crossings before its own
-// (32 crossings ranked at a time, no limit on their number).  Counts the events,
-// or writes them to `out` (EMIT).
-template <bool EMIT>
-__device__ __noinline__ uint32_t crowded(const RowScan &r, const int4 *edges, const uint32_t *ends, uint32_t *out) {
+// Sorts v[0 .. n) by a whole warp: bitonic, every exchange towards ascending
+// order (each merge starts with mirrored pairs), so entries past n need not exist.
+__device__ __forceinline__ void sort_list(uint32_t *v, uint32_t n) {
     const uint32_t lane = threadIdx.x & 31u;
+    for (uint32_t k = 2; (k >> 1) < n; k <<= 1)
+        for (uint32_t j = k >> 1; j; j >>= 1) {
+            for (uint32_t q = lane;; q += 32u) {
+                const uint32_t lo = ((q & ~(j - 1u)) << 1) | (q & (j - 1u));
+                const uint32_t hi = j == k >> 1 ? lo ^ (k - 1u) : lo + j;
+                if (lo >= n) break;
+                if (hi >= n) continue;
+                const uint32_t a = v[lo], b = v[hi];
+                if (a > b) {
+                    v[lo] = b;
+                    v[hi] = a;
+                }
+            }
+            __syncwarp();
+        }
+}
+
+// A sub-scanline with more crossings than a column holds, by a whole warp in
+// global memory: `v` holds nb + 1 words, the most events the sub-scanline can
+// have.  The keys go to v[1 ..], are sorted there, and are walked 32 at a time
+// into events from v[0] on (never past the keys read).  Returns their number.
+// n log^2 n / 32 steps, whatever the crossings: ties and shared pixels are usual
+// where contours are clipped.
+__device__ __noinline__ uint32_t crowded(const RowScan &r, const int4 *edges, const uint32_t *ends, uint32_t *v) {
+    const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
     const uint32_t psh = r.kind == 2u ? 0u : 2u, lm = r.kind == 2u ? 0u : 3u;
     const uint32_t *tab = ends + 16 * r.kind;
-    auto key_at = [&](uint32_t j, uint32_t *key) {
-        return crossing_key(__ldg(edges + __ldg(r.list + j)), r.y, r.base, r.xmax, key);
-    };
-    auto winding_before = [&](uint32_t key, uint32_t i) {
-        int32_t w = 0;
-        for (uint32_t j = 0; j < r.nb; j++) {
-            uint32_t kj;
-            if (key_at(j, &kj) && (kj < key || (kj == key && j < i))) w += key_winding(kj);
-        }
-        return w;
-    };
-    uint32_t count = 0;
-    for (uint32_t i0 = 0; i0 < r.nb; i0 += 32) {
-        const uint32_t i = i0 + lane;
+    uint32_t n = 0;
+    int32_t w = 0;
+    for (uint32_t i0 = 0; i0 < r.nb; i0 += 32u) {
         uint32_t key = 0;
-        bool end = false, in = false;
-        if (i < r.nb && key_at(i, &key)) {
-            const int32_t w = winding_before(key, i);
-            in = (w & r.fill_mask) != 0;
-            end = in != (((w + key_winding(key)) & r.fill_mask) != 0);
+        const bool in = i0 + lane < r.nb &&
+                        crossing_key(__ldg(edges + __ldg(r.list + i0 + lane)), r.y, r.base, r.xmax, &key, &w);
+        const uint32_t who = __ballot_sync(0xffffffffu, in);
+        if (in) v[1u + n + (uint32_t)__popc(who & below)] = key;
+        n += (uint32_t)__popc(who);
+    }
+    w = __reduce_add_sync(0xffffffffu, w);
+    __syncwarp();
+    sort_list(v + 1, n);
+    uint32_t m = 0, left = 0;  // events, and where the last span opened
+    if ((w & r.fill_mask) != 0) {  // open at the row's start
+        if (lane == 0) v[0] = r.off + tab[0];
+        m = 1;
+    }
+    for (uint32_t i0 = 0; i0 < n; i0 += 32u) {
+        const bool valid = i0 + lane < n;
+        const uint32_t key = valid ? v[1u + i0 + lane] : 0u;
+        int32_t upto = valid ? key_winding(key) : 0;
+        const int32_t own = upto;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int32_t t = __shfl_up_sync(0xffffffffu, upto, o);
+            if (lane >= (uint32_t)o) upto += t;
         }
-        const uint32_t who = __ballot_sync(0xffffffffu, end);
-        if (EMIT && end) {
-            const uint32_t x = key_sub(key), p = x >> psh;
-            uint32_t t = x & lm;
-            if (in) {
-                // the span's opening end, if it lies in the same pixel: the last
-                // opening crossing before this one there
-                bool found = false;
-                uint32_t best = 0, best_j = 0;
-                if (r.kind == 1u)
-                    for (uint32_t j = 0; j < r.nb; j++) {
-                        uint32_t kj;
-                        if (!key_at(j, &kj) || !(kj < key || (kj == key && j < i)) || (key_sub(kj) >> 2) != p) continue;
-                        if (found && (kj < best || (kj == best && j < best_j))) continue;
-                        const int32_t wj = winding_before(kj, j);
-                        if ((wj & r.fill_mask) != 0 || ((wj + key_winding(kj)) & r.fill_mask) == 0) continue;
-                        found = true;
-                        best = kj;
-                        best_j = j;
-                    }
-                t += found && (key_sub(best) & 3u) != 0u ? 12u : 4u;
-            }
-            out[count + (uint32_t)__popc(who & ((1u << lane) - 1u))] = (r.off + p) + tab[t];
-        }
-        count += (uint32_t)__popc(who);
+        upto += w;
+        const bool in = ((upto - own) & r.fill_mask) != 0, now = (upto & r.fill_mask) != 0, end = valid && in != now;
+        const uint32_t who = __ballot_sync(0xffffffffu, end), opens = __ballot_sync(0xffffffffu, end && now);
+        const uint32_t x = key_sub(key), p = x >> psh, mine = opens & below;
+        const uint32_t opened = __shfl_sync(0xffffffffu, x, mine ? 31 - __clz(mine) : 0), from = mine ? opened : left;
+        uint32_t t = x & lm;
+        if (in) t += ((from & lm) != 0u && (from >> psh) == p) ? 12u : 4u;
+        __syncwarp();  // these 32 keys have been read
+        if (end) v[m + (uint32_t)__popc(who & below)] = (r.off + p) + tab[t];
+        m += (uint32_t)__popc(who);
+        w = __shfl_sync(0xffffffffu, upto, 31);
+        if (opens) left = __shfl_sync(0xffffffffu, x, 31 - __clz(opens));
+    }
+    if ((w & r.fill_mask) != 0) {  // unclosed: the span runs to the row's end
+        if (lane == 0) v[m] = (r.off + (r.xmax >> (16 + psh))) + tab[4];
+        m++;
     }
     __syncwarp();
-    if ((winding_before(0xFFFFFFFFu, 0) & r.fill_mask) != 0) {  // unclosed: the span runs to the row's end
-        if (EMIT && lane == 0) out[count] = (r.off + (r.xmax >> (16 + psh))) + tab[4];
-        count++;
-    }
-    return count;
+    return m;
 }
 
 __device__ __forceinline__ void cmp_swap(uint32_t &a, uint32_t &b) {
@@ -169,31 +193,36 @@ __device__ __forceinline__ void sort_column(uint32_t *col, uint32_t n) {
 __device__ __forceinline__ uint32_t lane_events(uint32_t *col, const RowScan &r, const int4 *edges, const uint32_t *ends,
                                                 uint32_t *first, uint32_t *last) {
     uint32_t n = 0;
+    int32_t w = 0;
+    uint32_t *keys = col + kColStride;  // from the second entry on: the walk writes one event ahead
 #pragma unroll 4
     for (uint32_t i = 0; i < r.nb; i++) {
         const int4 e = __ldg(edges + __ldg(r.list + i));
         uint32_t key;
-        if (crossing_key(e, r.y, r.base, r.xmax, &key)) {
-            if (n < (uint32_t)kCol - 1) col[n * kColStride] = key;
+        if (crossing_key(e, r.y, r.base, r.xmax, &key, &w)) {
+            if (n < (uint32_t)kMaxSort) keys[n * kColStride] = key;
             n++;
         }
     }
-    const bool over = n > (uint32_t)kCol - 1;
+    const bool over = n > (uint32_t)kMaxSort;
     if (over) n = 0;
     const uint32_t most = __reduce_max_sync(0xffffffffu, n);
-    if (most > 16) sort_column<32>(col, n);
-    else if (most > 8) sort_column<16>(col, n);
-    else if (most > 4) sort_column<8>(col, n);
-    else if (most > 1) sort_column<4>(col, n);
+    if (most > 16) sort_column<kMaxSort>(keys, n);
+    else if (most > 8) sort_column<16>(keys, n);
+    else if (most > 4) sort_column<8>(keys, n);
+    else if (most > 1) sort_column<4>(keys, n);
     // walk: each end of a span overwrites the column from its start (never past
     // the crossings read)
     const uint32_t psh = r.kind == 2u ? 0u : 2u, lm = r.kind == 2u ? 0u : 3u;
     const uint32_t *tab = ends + 16 * r.kind;
     uint32_t m = 0, left = 0, f = 0;
-    int32_t w = 0;
-    bool in = false;  // inside a span
+    bool in = (w & r.fill_mask) != 0;  // inside a span
+    if (in) {  // open at the row's start
+        col[0] = r.off + tab[0];
+        m = 1;
+    }
     for (uint32_t i = 0; i < n; i++) {
-        const uint32_t key = col[i * kColStride];
+        const uint32_t key = keys[i * kColStride];
         w += key_winding(key);
         const bool now = (w & r.fill_mask) != 0;
         if (now != in) {
@@ -301,9 +330,16 @@ k_events(const StreamRec *streams, uint32_t nstreams, uint32_t ntasks, const Dra
                 s.fill_mask = __shfl_sync(0xffffffffu, r.fill_mask, src);
                 return s;
             };
+            // each sub-scanline of a row has a quarter of the row's room in the list,
+            // where a crowded one makes its events
+            uint32_t *list = events + 4ull * ((unsigned long long)boff + slot);
+            auto list_of = [&](int src) {
+                return reinterpret_cast<uint32_t *>(__shfl_sync(0xffffffffu, (unsigned long long)(uintptr_t)list, src));
+            };
             for (uint32_t o = overs; o; o &= o - 1u) {
                 const int src = __ffs(o) - 1;
-                const uint32_t c = crowded<false>(scan_of(src), edges, ends, nullptr);
+                const RowScan s = scan_of(src);
+                const uint32_t c = crowded(s, edges, ends, list_of(src) + (size_t)(src & 3) * (s.nb + 1u));
                 if ((int)lane == src) m = c;
             }
             // the row's header and the lanes' places in its list
@@ -323,7 +359,6 @@ k_events(const StreamRec *streams, uint32_t nstreams, uint32_t ntasks, const Dra
                 else if (all) h = all << 20 | (first >> 5) << 10 | last >> 5;
                 headers[slot] = h;
             }
-            uint32_t *list = events + 4ull * ((unsigned long long)boff + slot);
             // each row's list as a run: entry k is entry k - before of the lane
             // whose share holds it
             for (int g = 0; g < 32; g += 4) {
@@ -331,17 +366,31 @@ k_events(const StreamRec *streams, uint32_t nstreams, uint32_t ntasks, const Dra
                 if (!n) continue;
                 const uint32_t s1 = __shfl_sync(0xffffffffu, before, g + 1), s2 = __shfl_sync(0xffffffffu, before, g + 2),
                                s3 = __shfl_sync(0xffffffffu, before, g + 3);
-                uint32_t *dst = reinterpret_cast<uint32_t *>(
-                    __shfl_sync(0xffffffffu, (unsigned long long)(uintptr_t)list, g));
+                uint32_t *dst = list_of(g);
                 const uint32_t og = overs >> g & 0xFu;
-                for (uint32_t k = lane; k < n; k += 32u) {
-                    const uint32_t s = (uint32_t)(k >= s1) + (uint32_t)(k >= s2) + (uint32_t)(k >= s3);
-                    const uint32_t i = k - (s == 0u ? 0u : s == 1u ? s1 : s == 2u ? s2 : s3);
-                    if (!(og >> s & 1u)) dst[k] = cols[warp][i * kColStride + (uint32_t)g + s];
+                if (og == 0u) {
+                    for (uint32_t k = lane; k < n; k += 32u) {
+                        const uint32_t s = (uint32_t)(k >= s1) + (uint32_t)(k >= s2) + (uint32_t)(k >= s3);
+                        const uint32_t i = k - (s == 0u ? 0u : s == 1u ? s1 : s == 2u ? s2 : s3);
+                        dst[k] = cols[warp][i * kColStride + (uint32_t)g + s];
+                    }
+                    continue;
                 }
-                for (uint32_t o = og; o; o &= o - 1u) {
-                    const int s = __ffs(o) - 1;
-                    crowded<true>(scan_of(g + s), edges, ends, dst + (s == 0 ? 0u : s == 1 ? s1 : s == 2 ? s2 : s3));
+                // sub-scanlines in order: a share never starts after its own
+                // quarter, so it overwrites no later one
+                for (int s = 0; s < 4; s++) {
+                    const uint32_t from = s == 0 ? 0u : s == 1 ? s1 : s == 2 ? s2 : s3;
+                    const uint32_t c = (s == 0 ? s1 : s == 1 ? s2 : s == 2 ? s3 : n) - from;
+                    const uint32_t room = __shfl_sync(0xffffffffu, r.nb, g + s) + 1u;
+                    const uint32_t *src = dst + (size_t)s * room;
+                    for (uint32_t k0 = 0; k0 < c; k0 += 32u) {
+                        const uint32_t k = k0 + lane;
+                        uint32_t e = 0;
+                        if (k < c) e = (og >> s & 1u) ? src[k] : cols[warp][k * kColStride + (uint32_t)(g + s)];
+                        __syncwarp();
+                        if (k < c) dst[from + k] = e;
+                        __syncwarp();
+                    }
                 }
             }
             __syncwarp();  // the columns have been read

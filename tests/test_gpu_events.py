@@ -90,3 +90,51 @@ def test_spans_inside_one_pixel(gpu, oracle_mod):
                       [x, 0, x + d, 0, x + d, 8, x, 8, x + d, 0, x + d + 0.5, 0, x + d + 0.5, 8, x + d, 8],
                       A.EVENODD if k % 3 else A.NONZERO, 1))
     _check(oracle_mod, _tree(40, 8, paths), 40, 8)
+
+
+def _contours(xs, widths, h, tilt=0.0):
+    v, p = [], []
+    for x, d in zip(xs, widths):
+        v += [A.MOVE, A.LINE, A.LINE, A.LINE, A.CLOSE]
+        p += [x, 0.0, x + d, 0.0, x + d + tilt, h, x + tilt, h]
+    return v, p
+
+
+@pytest.mark.parametrize("aa", [1, 0])
+@pytest.mark.parametrize("rule", [A.NONZERO, A.EVENODD])
+@pytest.mark.parametrize("count", [15, 16, 31, 301, 700])
+def test_contours_beside_the_canvas(gpu, oracle_mod, count, rule, aa):
+    """A view into a drawing: most contours lie left or right of the canvas (their
+    edges run along the clip's sides), some reach into it, and the left ones leave
+    a winding of zero or not."""
+    w, h = 90, 6
+    g = np.random.default_rng(count)
+    paths = []
+    for k in range(4):
+        xs = np.concatenate([g.uniform(-400, -2, size=count), g.uniform(w, w + 300, size=count // 2),
+                             g.uniform(-30, w - 5, size=3 + k)])
+        widths = np.concatenate([g.uniform(0.2, 1.5, size=count + count // 2), g.uniform(1, 50, size=3 + k)])
+        widths[::3] *= -1  # both directions
+        if k % 2:
+            xs = np.append(xs, -20.0)
+            widths = np.append(widths, 20.0 + 3.3 * k)
+        paths.append(_contours(xs, widths, float(h) - 0.3, tilt=0.4 * k) + (rule, aa))
+    _check(oracle_mod, _tree(w, h, paths), w, h)
+
+
+@pytest.mark.parametrize("aa", [1, 0])
+@pytest.mark.parametrize("rule", [A.NONZERO, A.EVENODD])
+@pytest.mark.parametrize("count", [16, 33, 64, 257, 4001])
+def test_crossings_that_share_pixels(gpu, oracle_mod, count, rule, aa):
+    """Hundreds of crossings of equal x, or within two pixels, on every
+    sub-scanline.  The time grows with n log^2 n: 8,002 of them are no second's work."""
+    import time
+    w, h = 70, 3
+    g = np.random.default_rng(count)
+    same = _contours([20.125] * count, [7.25 + (rule == A.EVENODD and count % 2) * 0.5] * count, 3.0)
+    near = _contours(33.0 + np.round(g.uniform(0, 2, size=count) * 16) / 16, g.uniform(0.05, 0.5, size=count), 2.7)
+    tree = _tree(w, h, [same + (rule, aa), near + (rule, aa)])
+    R.render(tree, IDENT, w, h)
+    t0 = time.perf_counter()
+    _check(oracle_mod, tree, w, h)
+    assert time.perf_counter() - t0 < 20.0
