@@ -111,6 +111,11 @@ const char *rgpu_last_warning(void);
  * resvg::render (crates/resvg/src/lib.rs:34) without host copies. */
 int rgpu_render_device(const resvg_render_tree *tree, resvg_transform transform, uint32_t width, uint32_t height,
                        uint8_t *device_pixmap, uint32_t stride, void *stream);
+/* Working memory of every render: 20 bytes per (edge, row it crosses) and 28 per
+ * (row, draw of its surface), kept between calls (rgpu_trim releases it).  A
+ * submission that needs more than a third of the device's memory, or than could
+ * be allocated, is rendered in several passes over its rows, so its size is
+ * bounded by its records alone. */
 /* Batched form: renders `count` independent trees.  pixmaps[i] are DEVICE
  * pointers of widths[i]*heights[i]*4 bytes, cleared to transparent by the
  * caller or not (rendering draws onto content).  One submission; the work is
@@ -188,9 +193,12 @@ int rgpu_set_wait_limit(uint32_t rounds);
  * the pixmap untouched);
  * rgpu_test_scan runs the device's exclusive prefix sum over `count` host words
  * (`offsets` and `total` are host words too; a total of 2^32 - 1 or more is
- * reported as 2^32 - 1, and the offsets are then unspecified). */
+ * reported as 2^32 - 1, and the offsets are then unspecified);
+ * rgpu_test_pass_bytes(n) bounds a render pass's working memory to n bytes for
+ * submissions made afterwards (0 = the default). */
 int rgpu_test_withhold_window(int enabled);
 int rgpu_test_fail_allocations(uint32_t count);
+int rgpu_test_pass_bytes(uint64_t bytes);
 int rgpu_test_scan(const uint32_t *counts, uint32_t count, uint32_t *offsets, uint32_t *total);
 /* rgpu_render_batch cuts a batch into chunks of about equal estimated cost
  * (pixels x paths) and flattens and uploads chunk k + 1 on the host while the

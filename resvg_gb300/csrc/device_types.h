@@ -180,11 +180,12 @@ struct StreamRec {
     uint32_t out_stride;           // bytes per row
     uint64_t out_ptr;              // device pointer of the target surface
     uint32_t task_off;             // first task of the event kernel: 32 draws of one row each
-    uint32_t bin_off;              // slots (row, draw) of this stream: bin_off + row * draw_cnt + draw - draw_off
+    uint32_t bin_off;              // slots (row, draw) of this stream: bin_off + (row - row_lo) * draw_cnt + draw - draw_off
     uint32_t max_depth;            // layer-stack depth needed
     int32_t surface;               // internal surface rendered into (filter content), or -1
     uint32_t level;                // dependency level: content streams render before their parents
     uint32_t row_w;                // widest work item, a power of two: 64 .. kRasterMaxRow
+    int32_t row_lo, row_hi;        // the rows of one pass (all of them where a submission takes one pass)
 };
 constexpr uint32_t kRasterMaxRow = 512;
 

@@ -67,11 +67,15 @@ struct DevBuf {
         if (p) cudaFree(p);
         p = nullptr;
         cap = 0;
-        size_t want = std::max(bytes, (size_t)4096);
-        want = want + want / 4;
+        // a quarter of room to grow, of large ones at most 256 MB
+        const size_t want = std::max(bytes, (size_t)4096) + std::min(bytes / 4, (size_t)256 << 20);
         if (forced_alloc_failure()) return cudaErrorMemoryAllocation;
         cudaError_t e = cudaMalloc(&p, want);
         if (e == cudaSuccess) cap = want;
+        else {
+            p = nullptr;
+            cudaGetLastError();  // reported here, not by the next launch
+        }
         return e;
     }
     template <class T> T *as() const { return (T *)p; }
@@ -159,17 +163,42 @@ struct BufScratch : FilterScratch {
 constexpr uint32_t kPipeMinScenes = 64;
 constexpr uint32_t kPipeChunks = 8;
 
+// The bins, events and slots of a submission's rows live in buffers of bounded
+// size: a submission that needs more is rendered in several passes over its rows
+// (and its streams), each binned, turned into events and rasterised by itself.
+// A binned edge takes 20 bytes (its index, 4 event words), a slot 28 (count,
+// offset, header, 4 event words).
+// The bound is a third of the device's memory (Context::pass_bytes), or what is
+// left of it when an allocation fails.  Smaller passes cost time, as each reads
+// all edges twice and ends with SMs that wait for the last rows: 4,096 mixed
+// scenes, 77 GB, take 750 ms in one pass, 765 bounded to 48 GB, 782 to 24, 828 to 8.
+constexpr uint64_t kBinnedBytes = 20, kSlotBytes = 28;
+
+// One pass: some rows of some streams.  The only pass of a submission holds all
+// dependency levels; where there are several, each is of one level.
+struct Pass {
+    uint32_t level0 = 0, level1 = 0;  // levels rasterised
+    bool last = true;                 // nothing of these levels is left after it
+    uint32_t streams = 0;             // the pass's records of all streams, from this one of Plan::streams on
+    uint64_t nslots = 0, ntasks = 0;  // (row, draw) slots; tasks of the event kernel
+    uint32_t nbinned = 0;             // binned edges (known after the sizing run)
+    std::vector<uint32_t> item_off, item_cnt;  // work items per level, from level0 on
+};
+
 // A flattened submission with its work decomposition.
 struct Plan {
     SceneBuild sb;
     std::vector<WorkItem> items;
-    std::vector<uint32_t> level_off, level_cnt;  // work items per dependency level
+    std::vector<Pass> passes;
+    std::vector<StreamRec> streams;   // of all passes
+    uint64_t slot_budget = 0;         // slots of a pass, at most (0: by the context's bound)
     uint32_t row_w = 64;    // widest work-item row
-    uint64_t nbins = 0;      // (row, draw) slots
-    uint64_t ntasks = 0;     // of the event kernel
+    uint64_t nbins = 0;      // (row, draw) slots of the largest pass
+    uint32_t raster_launches = 0;
     uint32_t max_depth = 1;
     uint32_t grid = 1;
-    uint32_t nedges = 0, nbinned = 0;  // known after the first (sizing) run
+    uint32_t nedges = 0;     // known after the first (sizing) run
+    uint64_t nbinned = 0;    // of all passes, likewise
     // segment slots and transformed points: the build's own counts, or with
     // device-stroked paths the device's totals (known after the sizing run)
     uint64_t nsegs = 0, ntpts = 0;
@@ -222,6 +251,8 @@ struct Context {
     std::mutex mu;
     int device = -1;
     int sms = 0;
+    uint64_t pass_bytes = 0;     // working memory of a pass, at most
+    uint64_t device_bytes = 0;
     cudaStream_t stream = nullptr;
     RasterTimer timer;
     Buffers buf;
@@ -282,6 +313,8 @@ int ensure_device(Context &c) {
         return RGPU_ERR_NO_DEVICE;
     }
     c.sms = prop.multiProcessorCount;
+    c.device_bytes = prop.totalGlobalMem;
+    if (!c.pass_bytes) c.pass_bytes = c.device_bytes / 3;
     CK(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
     CK(raster_init());
     CK(stroke_warmup(c.stream));
@@ -388,6 +421,133 @@ int layout_strokes(Plan &p) {
     return RGPU_OK;
 }
 
+// Fills a pass's stream records and work items from its streams' row ranges
+// (row_lo and row_hi of the records; no rows: not in the pass).
+void plan_items(Plan &p, Pass &ps, size_t nstreams) {
+    StreamRec *recs = p.streams.data() + ps.streams;
+    ps.nslots = ps.ntasks = 0;
+    for (size_t si = 0; si < nstreams; si++) {
+        StreamRec &st = recs[si];
+        const uint64_t rows = (uint64_t)(st.row_hi - st.row_lo);
+        st.bin_off = (uint32_t)ps.nslots;
+        ps.nslots += rows * st.draw_cnt;
+        st.task_off = (uint32_t)ps.ntasks;
+        ps.ntasks += rows * ((st.draw_cnt + 31) / 32);
+    }
+    ps.item_off.assign(ps.level1 - ps.level0 + 1, 0);
+    ps.item_cnt.assign(ps.level1 - ps.level0 + 1, 0);
+    for (uint32_t lv = ps.level0; lv <= ps.level1; lv++) {
+        const size_t first = p.items.size();
+        for (uint32_t si = 0; si < nstreams; si++) {
+            const StreamRec &st = recs[si];
+            if (st.level != lv) continue;
+            // rows wider than row_w in pieces of about equal width
+            const int32_t np = (st.out_w + (int32_t)st.row_w - 1) / (int32_t)st.row_w;
+            const int32_t cw = ((st.out_w + np - 1) / np + 31) & ~31;
+            for (int32_t y = st.row_lo; y < st.row_hi; y++)
+                for (int32_t x0 = 0; x0 < st.out_w; x0 += cw)
+                    p.items.push_back(WorkItem{si, (uint32_t)y, x0, std::min(x0 + cw, st.out_w)});
+        }
+        ps.item_off[lv - ps.level0] = (uint32_t)first;
+        ps.item_cnt[lv - ps.level0] = (uint32_t)(p.items.size() - first);
+        // the persistent kernel takes items in order: heaviest first (draws x
+        // pixels) shortens the tail when scenes of very different cost share
+        // a launch
+        auto cost = [&](const WorkItem &it) {
+            const StreamRec &st = recs[it.stream];
+            return (uint64_t)st.draw_cnt * (uint64_t)(it.x1 - it.x0);
+        };
+        std::stable_sort(p.items.begin() + first, p.items.end(),
+                         [&](const WorkItem &a, const WorkItem &b) { return cost(a) > cost(b); });
+    }
+}
+
+// Cuts the submission into passes of at most slot_budget slots (or one row of
+// one stream each) and lists their work items.
+int plan_passes(Context &c, Plan &p) {
+    SceneBuild &sb = p.sb;
+    const size_t ns = sb.streams.size();
+    if (!p.slot_budget) p.slot_budget = c.pass_bytes / kSlotBytes;
+    const uint64_t budget = std::min<uint64_t>(p.slot_budget, 0xF0000000ull);  // slots are counted in 32 bits
+    p.items.clear();
+    p.passes.clear();
+    p.streams.clear();
+    uint64_t total = 0;
+    for (const StreamRec &st : sb.streams) total += (uint64_t)st.out_h * st.draw_cnt;
+    auto open = [&](uint32_t lv0, uint32_t lv1) {
+        Pass ps;
+        ps.level0 = lv0;
+        ps.level1 = lv1;
+        ps.streams = (uint32_t)p.streams.size();
+        p.streams.insert(p.streams.end(), sb.streams.begin(), sb.streams.end());
+        for (size_t si = 0; si < ns; si++) p.streams[ps.streams + si].row_lo = p.streams[ps.streams + si].row_hi = 0;
+        p.passes.push_back(ps);
+    };
+    if (total <= budget) {
+        open(0, sb.max_level);
+        for (size_t si = 0; si < ns; si++) p.streams[si].row_hi = p.streams[si].out_h;
+        plan_items(p, p.passes.back(), ns);
+    } else {
+        for (uint32_t lv = 0; lv <= sb.max_level; lv++) {
+            uint64_t used = 0;
+            open(lv, lv);
+            for (size_t si = 0; si < ns; si++) {
+                const StreamRec &st = sb.streams[si];
+                if (st.level != lv) continue;
+                for (int32_t y = 0; y < st.out_h;) {
+                    const uint64_t left = budget > used ? budget - used : 0;
+                    int64_t rows = st.draw_cnt ? (int64_t)(left / st.draw_cnt) : st.out_h;
+                    if (rows < 1 && used) {  // the pass is full
+                        p.passes.back().last = false;
+                        plan_items(p, p.passes.back(), ns);
+                        open(lv, lv);
+                        used = 0;
+                        continue;
+                    }
+                    rows = std::min<int64_t>(std::max<int64_t>(rows, 1), st.out_h - y);
+                    StreamRec &rec = p.streams[p.passes.back().streams + si];
+                    rec.row_lo = y;
+                    rec.row_hi = y + (int32_t)rows;
+                    used += (uint64_t)rows * st.draw_cnt;
+                    y += (int32_t)rows;
+                    if (y < st.out_h) used = std::max(used, budget);  // a stream has one run of rows in a pass
+                }
+            }
+            plan_items(p, p.passes.back(), ns);
+        }
+    }
+    p.nbins = 0;
+    p.raster_launches = 0;
+    uint32_t most = 1;
+    for (const Pass &ps : p.passes) {
+        p.nbins = std::max(p.nbins, ps.nslots);
+        for (uint32_t n : ps.item_cnt) {
+            most = std::max(most, n);
+            p.raster_launches += n ? 1 : 0;
+        }
+    }
+    if (p.nbins > 0xF0000000ull) { set_error("a row holds too many draws"); return RGPU_ERR_CAPACITY; }
+    uint32_t per_sm = (uint32_t)raster_max_blocks_per_sm(p.row_w);
+    p.grid = std::max<uint32_t>(1, std::min<uint32_t>(most, (uint32_t)c.sms * per_sm));
+    return RGPU_OK;
+}
+
+// Smaller passes than the present ones; false where every pass is one row already.
+bool shrink_passes(Plan &p, double factor) {
+    uint64_t rows = 0;
+    for (const Pass &ps : p.passes) {
+        uint64_t n = 0;
+        for (size_t si = 0; si < p.sb.streams.size(); si++) {
+            const StreamRec &st = p.streams[ps.streams + si];
+            n += st.draw_cnt ? (uint64_t)(st.row_hi - st.row_lo) : 0;
+        }
+        rows = std::max(rows, n);
+    }
+    if (rows <= 1) return false;
+    p.slot_budget = std::max<uint64_t>(1, (uint64_t)((double)std::min(p.slot_budget, p.nbins) * std::min(factor, 0.75)));
+    return true;
+}
+
 int plan_scene(Context &c, Plan &p) {
     SceneBuild &sb = p.sb;
     if (sb.stroke_jobs.empty()) {
@@ -429,8 +589,6 @@ int plan_scene(Context &c, Plan &p) {
         int r = layout_strokes(p);
         if (r) return r;
     }
-    p.row_w = 64;
-    p.items.clear();
     // the raster kernel finds a fill's paint and gradient through its command
     for (Cmd &cmd : sb.cmds)
         if (cmd.op == CMD_FILL || cmd.op == CMD_APPLY_REGION) {
@@ -439,49 +597,17 @@ int plan_scene(Context &c, Plan &p) {
             const uint32_t g = pr.kind == 1 ? pr.grad : 0xFFFFFFFFu;
             std::memcpy(&cmd.f, &g, 4);
         }
-    p.nbins = p.ntasks = 0;
+    p.row_w = 64;
     p.max_depth = 1;
     std::vector<uint32_t> level_w(sb.max_level + 1);
     for (uint32_t lv = 0; lv <= sb.max_level; lv++) level_w[lv] = pick_row_w(sb, lv, c.tuning);
-    for (uint32_t si = 0; si < sb.streams.size(); si++) {
-        StreamRec &st = sb.streams[si];
+    for (StreamRec &st : sb.streams) {
         st.row_w = level_w[st.level];
         p.row_w = std::max(p.row_w, st.row_w);
-        st.bin_off = (uint32_t)p.nbins;
-        p.nbins += (uint64_t)st.out_h * st.draw_cnt;
-        st.task_off = (uint32_t)p.ntasks;
-        p.ntasks += (uint64_t)st.out_h * ((st.draw_cnt + 31) / 32);
         p.max_depth = std::max(p.max_depth, st.max_depth + 1);
     }
-    p.level_off.assign(sb.max_level + 1, 0);
-    p.level_cnt.assign(sb.max_level + 1, 0);
-    for (uint32_t lv = 0; lv <= sb.max_level; lv++) {
-        p.level_off[lv] = (uint32_t)p.items.size();
-        for (uint32_t si = 0; si < sb.streams.size(); si++) {
-            const StreamRec &st = sb.streams[si];
-            if (st.level != lv) continue;
-            // rows wider than row_w in pieces of about equal width
-            const int32_t np = (st.out_w + (int32_t)st.row_w - 1) / (int32_t)st.row_w;
-            const int32_t cw = ((st.out_w + np - 1) / np + 31) & ~31;
-            for (uint32_t y = 0; y < (uint32_t)st.out_h; y++)
-                for (int32_t x0 = 0; x0 < st.out_w; x0 += cw)
-                    p.items.push_back(WorkItem{si, y, x0, std::min(x0 + cw, st.out_w)});
-        }
-        p.level_cnt[lv] = (uint32_t)p.items.size() - p.level_off[lv];
-        // the persistent kernel takes items in order: heaviest first (draws x
-        // pixels) shortens the tail when scenes of very different cost share
-        // a launch
-        auto cost = [&](const WorkItem &it) {
-            const StreamRec &st = sb.streams[it.stream];
-            return (uint64_t)st.draw_cnt * (uint64_t)(it.x1 - it.x0);
-        };
-        std::stable_sort(p.items.begin() + p.level_off[lv], p.items.end(),
-                         [&](const WorkItem &a, const WorkItem &b) { return cost(a) > cost(b); });
-    }
-    if (p.nbins > 0xF0000000ull) { set_error("too many (row, draw) slots"); return RGPU_ERR_CAPACITY; }
-    uint32_t per_sm = (uint32_t)raster_max_blocks_per_sm(p.row_w);
-    p.grid = std::max<uint32_t>(1, std::min<uint32_t>((uint32_t)p.items.size(), (uint32_t)c.sms * per_sm));
-    return RGPU_OK;
+    p.slot_budget = 0;
+    return plan_passes(c, p);
 }
 
 int ensure_stroke_buffers(Buffers &b, Plan &p) {
@@ -510,6 +636,29 @@ int ensure_segment_buffers(Buffers &b, Plan &p) {
     CK(b.seg_counts.ensure((nsegs + 1) * 4));
     CK(b.seg_offsets.ensure((nsegs + 1) * 4));
     CK(b.scan_scratch.ensure(scan_scratch_words(std::max<uint64_t>({nsegs + 1, p.nbins + 1, p.sb.draws.size() + 1})) * 4));
+    return RGPU_OK;
+}
+
+// The buffers of a pass's slots; where memory is short, passes are made smaller.
+int ensure_slot_buffers(Context &c, Buffers &b, Plan &p) {
+    for (;;) {
+        const size_t bytes = (p.nbins + 1) * 4;
+        cudaError_t e = b.bin_counts.ensure(bytes);
+        if (e == cudaSuccess) e = b.bin_offsets.ensure(bytes);
+        if (e == cudaSuccess) e = b.headers.ensure(bytes);
+        if (e != cudaErrorMemoryAllocation || !shrink_passes(p, 0.5)) {
+            CK(e);
+            return RGPU_OK;
+        }
+        int r = plan_passes(c, p);
+        if (r) return r;
+    }
+}
+
+// What the raster launches of the present passes need besides their records.
+int ensure_raster_buffers(Buffers &b, Plan &p) {
+    CK(b.stack.ensure((size_t)p.grid * raster_warps() * p.max_depth * p.row_w * 4));
+    CK(b.counter.ensure(4 * std::max<size_t>(p.raster_launches, 1)));
     return RGPU_OK;
 }
 
@@ -682,6 +831,9 @@ int upload_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, HostBuf *stagin
         if (st.surface >= 0) st.out_ptr = (uint64_t)(uintptr_t)b.surf[st.surface].p;
     for (auto &L : sb.layers)
         if (L.surf >= 0) L.buf = (uint64_t)(uintptr_t)b.surf[L.surf].p;
+    int r;
+    if ((r = ensure_slot_buffers(c, b, p))) return r;
+    for (size_t i = 0; i < p.streams.size(); i++) p.streams[i].out_ptr = sb.streams[i % sb.streams.size()].out_ptr;
     for (const auto &q : sb.patterns) {
         ImageRec im{(uint64_t)(uintptr_t)b.surf[q.shade].p, q.bx, q.by, q.bw, q.bh};
         std::memcpy(&sb.grads[q.grad], &im, sizeof(im));
@@ -690,13 +842,12 @@ int upload_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, HostBuf *stagin
     size_t stage = rup(sb.verbs.size()) + rup(sb.pts.size() * 4) + rup(sb.draws.size() * sizeof(DrawRec)) +
                    rup(sb.paints.size() * sizeof(PaintRec)) + rup(sb.grads.size() * sizeof(GradRec)) +
                    rup(sb.layers.size() * sizeof(LayerRec)) + rup(sb.cmds.size() * sizeof(Cmd)) +
-                   rup(sb.streams.size() * sizeof(StreamRec)) + rup(p.items.size() * sizeof(WorkItem)) +
+                   rup(p.streams.size() * sizeof(StreamRec)) + rup(p.items.size() * sizeof(WorkItem)) +
                    rup(sb.hairs.size() * sizeof(HairRec)) + rup(sb.hair_spans.size() * sizeof(HairSpan)) +
                    rup(sb.stroke_jobs.size() * sizeof(StrokeJob)) +
                    rup(sb.dashes.size() * 4) + 4096;
     CK(staging.ensure(stage));
     size_t off = 0;
-    int r;
     if ((r = upload(staging, b.verbs, sb.verbs, off, s))) return r;
     if ((r = upload(staging, b.pts, sb.pts, off, s))) return r;
     if ((r = upload(staging, b.draws, sb.draws, off, s))) return r;
@@ -704,7 +855,7 @@ int upload_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, HostBuf *stagin
     if ((r = upload(staging, b.grads, sb.grads, off, s))) return r;
     if ((r = upload(staging, b.layers, sb.layers, off, s))) return r;
     if ((r = upload(staging, b.cmds, sb.cmds, off, s))) return r;
-    if ((r = upload(staging, b.streams, sb.streams, off, s))) return r;
+    if ((r = upload(staging, b.streams, p.streams, off, s))) return r;
     if ((r = upload(staging, b.items, p.items, off, s))) return r;
     if ((r = upload(staging, b.hairs, sb.hairs, off, s))) return r;
     if ((r = upload(staging, b.hair_spans, sb.hair_spans, off, s))) return r;
@@ -718,17 +869,79 @@ int upload_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, HostBuf *stagin
         if ((r = ensure_segment_buffers(b, p))) return r;
     CK(b.totals.ensure(64));
     CK(b.scan_scratch.ensure(scan_scratch_words(std::max<uint64_t>({p.nsegs + 1, p.nbins + 1, sb.draws.size() + 1})) * 4));
-    CK(b.bin_counts.ensure((p.nbins + 1) * 4));
-    CK(b.bin_offsets.ensure((p.nbins + 1) * 4));
-    CK(b.headers.ensure((p.nbins + 1) * 4));
-    CK(b.stack.ensure((size_t)p.grid * raster_warps() * p.max_depth * p.row_w * 4));
     CK(b.err.ensure(16));
-    CK(b.counter.ensure(4 * (sb.max_level + 1)));
+    return ensure_raster_buffers(b, p);
+}
+
+// kernels of a render of a sized plan (without filters): setup, edges twice, their
+// scan and the draws' edge ranges, and per pass the bins twice, their scan, the
+// events and one raster launch
+uint32_t plan_launches(const Plan &p) {
+    uint32_t n = 4 + scan_launches(p.nsegs + 1);
+    for (const Pass &ps : p.passes) n += 4 + scan_launches(ps.nslots + 1);
+    return n;
+}
+
+// The binned edges of every slot of a pass, and the places of its lists.
+int count_pass(Buffers &b, const Plan &p, const Pass &ps, cudaStream_t s) {
+    CK(cudaMemsetAsync(b.bin_counts.p, 0, (ps.nslots + 1) * 4, s));
+    CK(launch_bin(false, b.edges.as<EdgeRec>(), b.edge_draw.as<uint32_t>(), p.nedges, b.draws.as<DrawRec>(),
+                  b.streams.as<StreamRec>() + ps.streams, b.bin_counts.as<uint32_t>(), nullptr, 0, nullptr, nullptr, s));
+    CK(launch_exclusive_scan(b.bin_counts.as<uint32_t>(), b.bin_offsets.as<uint32_t>(), ps.nslots + 1,
+                             b.scan_scratch.as<uint32_t>(), b.totals.as<uint32_t>() + 1, s));
     return RGPU_OK;
 }
 
-// kernels of a render of a sized plan (without filters and further raster levels)
-uint32_t plan_launches(const Plan &p) { return 8 + scan_launches(p.nsegs + 1) + scan_launches(p.nbins + 1); }
+// The sizing run's second part: every pass's binned edges, and buffers for the
+// largest.  Passes that turn out larger than the bound, or than the memory there
+// is, are made smaller.  A single pass is left counted, in the buffers.
+int size_passes(Context &c, Buffers &b, Plan &p, cudaStream_t s) {
+    for (;;) {
+        double factor = 0.0;  // passes to be made smaller by it
+        uint64_t most = 0, words = 0;  // binned edges, and slots more, of the largest passes
+        p.nbinned = 0;
+        for (Pass &ps : p.passes) {
+            int r = count_pass(b, p, ps, s);
+            if (r) return r;
+            uint32_t tot = 0;
+            CK(cudaMemcpyAsync(&tot, b.totals.as<uint32_t>() + 1, 4, cudaMemcpyDeviceToHost, s));
+            CK(cudaStreamSynchronize(s));
+            const uint64_t bytes = kBinnedBytes * tot + kSlotBytes * ps.nslots;
+            const bool wraps = tot == 0xFFFFFFFFu;  // where the scan's total saturates: offsets are 32-bit
+            if (wraps || bytes > c.pass_bytes) {
+                factor = wraps ? 0.25 : 0.9 * (double)c.pass_bytes / (double)bytes;
+                if (shrink_passes(p, factor)) break;
+                if (wraps) {
+                    set_error("a row holds too many edges");
+                    return RGPU_ERR_CAPACITY;
+                }
+                factor = 0.0;
+            }
+            ps.nbinned = tot;
+            p.nbinned += tot;
+            most = std::max<uint64_t>(most, tot);
+            words = std::max<uint64_t>(words, tot + ps.nslots);
+        }
+        if (factor == 0.0) {
+            cudaError_t e = b.bins.ensure(std::max<uint64_t>(most, 1) * 4);
+            if (e == cudaSuccess) e = b.events.ensure((words + 1) * 16);
+            if (e != cudaErrorMemoryAllocation || !shrink_passes(p, 0.5)) {
+                CK(e);
+                return RGPU_OK;
+            }
+        }
+        int r = plan_passes(c, p);
+        if (!r) r = ensure_slot_buffers(c, b, p);
+        if (!r) r = ensure_segment_buffers(b, p);
+        if (!r) r = ensure_raster_buffers(b, p);
+        if (r) return r;
+        CK(b.streams.ensure(p.streams.size() * sizeof(StreamRec)));
+        CK(b.items.ensure(std::max<size_t>(p.items.size(), 1) * sizeof(WorkItem)));
+        CK(cudaMemcpyAsync(b.streams.p, p.streams.data(), p.streams.size() * sizeof(StreamRec), cudaMemcpyHostToDevice, s));
+        CK(cudaMemcpyAsync(b.items.p, p.items.data(), p.items.size() * sizeof(WorkItem), cudaMemcpyHostToDevice, s));
+        CK(cudaStreamSynchronize(s));
+    }
+}
 
 // Enqueues the device pipeline.  Without known sizes it synchronises twice to
 // read the edge and bin totals; with known sizes (a prepared scene rendered
@@ -764,34 +977,15 @@ int enqueue_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, RasterTimer *t
                     b.seg_counts.as<uint32_t>(), b.seg_offsets.as<uint32_t>(), b.edges.as<EdgeRec>(),
                     b.edge_draw.as<uint32_t>(), nedges, s));
     CK(launch_draw_edges(b.draws.as<DrawRec>(), ndraws, b.seg_offsets.as<uint32_t>(), s));
-    CK(cudaMemsetAsync(b.bin_counts.p, 0, (p.nbins + 1) * 4, s));
-    CK(launch_bin(false, b.edges.as<EdgeRec>(), b.edge_draw.as<uint32_t>(), nedges, b.draws.as<DrawRec>(),
-                  b.streams.as<StreamRec>(), b.bin_counts.as<uint32_t>(), nullptr, 0, nullptr, nullptr, s));
-    CK(launch_exclusive_scan(b.bin_counts.as<uint32_t>(), b.bin_offsets.as<uint32_t>(), p.nbins + 1,
-                             b.scan_scratch.as<uint32_t>(), totals + 1, s));
+    bool counted = false;
     if (!p.sized) {
-        uint32_t tot = 0;
-        CK(cudaMemcpyAsync(&tot, totals + 1, 4, cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        if (tot == 0xFFFFFFFFu) {  // where the scan's total saturates: bin offsets are 32-bit
-            set_error("the submission's rows hold too many edges: render fewer scenes at a time");
-            return RGPU_ERR_CAPACITY;
-        }
-        p.nbinned = tot;
-        CK(b.bins.ensure(std::max<uint32_t>(tot, 1) * 4ull));
-        CK(b.events.ensure(((uint64_t)tot + p.nbins + 1) * 16));
+        int r = size_passes(c, b, p, s);
+        if (r) return r;
+        counted = p.passes.size() == 1;
         p.sized = true;
     }
-    CK(cudaMemsetAsync(b.bin_counts.p, 0, (p.nbins + 1) * 4, s));
     CK(cudaMemsetAsync(b.err.p, 0, 4, s));
-    CK(launch_bin(true, b.edges.as<EdgeRec>(), b.edge_draw.as<uint32_t>(), nedges, b.draws.as<DrawRec>(),
-                  b.streams.as<StreamRec>(), b.bin_counts.as<uint32_t>(), b.bin_offsets.as<uint32_t>(), p.nbinned,
-                  b.err.as<uint32_t>(), b.bins.as<uint32_t>(), s));
-    CK(launch_events(b.streams.as<StreamRec>(), (uint32_t)sb.streams.size(), (uint32_t)p.ntasks, b.draws.as<DrawRec>(),
-                     b.edges.as<EdgeRec>(), b.bins.as<uint32_t>(), b.bin_offsets.as<uint32_t>(),
-                     b.bin_counts.as<uint32_t>(), b.headers.as<uint32_t>(), b.events.as<uint32_t>(),
-                     b.err.as<uint32_t>(), s));
-    CK(cudaMemsetAsync(b.counter.p, 0, 4 * (sb.max_level + 1), s));
+    CK(cudaMemsetAsync(b.counter.p, 0, 4 * std::max<size_t>(p.raster_launches, 1), s));
     for (const auto &st : sb.streams)
         if (st.surface >= 0) CK(cudaMemsetAsync(b.surf[st.surface].p, 0, (size_t)st.out_w * st.out_h * 4, s));
     BufScratch scratch(b);
@@ -799,36 +993,54 @@ int enqueue_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, RasterTimer *t
         CK(tm->ensure());
         tm->used = 0;
     }
-    for (uint32_t lv = 0; lv <= sb.max_level; lv++) {
-        const bool timed = tm && p.level_cnt[lv] && tm->used < RasterTimer::kPairs;
-        if (timed) CK(cudaEventRecord(tm->start[tm->used], s));
-        if (p.level_cnt[lv])
-            CK(launch_raster(p.row_w, p.grid, p.max_depth, b.streams.as<StreamRec>(),
-                             b.items.as<WorkItem>() + p.level_off[lv], p.level_cnt[lv], b.counter.as<uint32_t>() + lv,
-                             b.cmds.as<Cmd>(), b.draws.as<DrawRec>(), b.paints.as<PaintRec>(), b.grads.as<GradRec>(),
-                             b.layers.as<LayerRec>(), b.bin_offsets.as<uint32_t>(), b.headers.as<uint32_t>(),
-                             b.events.as<uint32_t>(), b.stack.as<uint32_t>(), b.hairs.as<HairRec>(),
-                             b.hair_spans.as<HairSpan>(), b.err.as<uint32_t>(), s));
-        if (timed) CK(cudaEventRecord(tm->stop[tm->used++], s));
-        for (const auto &q : sb.patterns) {
-            if (q.level != lv) continue;
-            const float inv[6] = {q.inv.sx, q.inv.ky, q.inv.kx, q.inv.sy, q.inv.tx, q.inv.ty};
-            CK(filter_pattern_shade(b.surf[q.tile].as<uint32_t>(), q.tw, q.th, (float *)b.surf[q.shade].p, q.bx, q.by,
-                                    q.bw, q.bh, inv, q.quality, q.repeat != 0, q.opacity, s));
+    uint32_t launch = 0;  // raster launches so far: each has an item counter
+    for (const Pass &ps : p.passes) {
+        if (!counted) {
+            int r = count_pass(b, p, ps, s);
+            if (r) return r;
         }
-        for (const auto &job : sb.jobs) {
-            if (job.level != lv) continue;
-            std::string ferr;
-            std::vector<FeImageSurface> ims;
-            for (uint32_t k = 0; k < job.image_count; k++) {
-                const FeImageReq &q = sb.fe_images[job.image_first + k];
-                ims.push_back(FeImageSurface{q.prim, b.surf[q.surface].as<uint32_t>()});
+        const StreamRec *streams = b.streams.as<StreamRec>() + ps.streams;
+        CK(cudaMemsetAsync(b.bin_counts.p, 0, (ps.nslots + 1) * 4, s));
+        CK(launch_bin(true, b.edges.as<EdgeRec>(), b.edge_draw.as<uint32_t>(), nedges, b.draws.as<DrawRec>(), streams,
+                      b.bin_counts.as<uint32_t>(), b.bin_offsets.as<uint32_t>(), ps.nbinned, b.err.as<uint32_t>(),
+                      b.bins.as<uint32_t>(), s));
+        CK(launch_events(streams, (uint32_t)sb.streams.size(), (uint32_t)ps.ntasks, b.draws.as<DrawRec>(),
+                         b.edges.as<EdgeRec>(), b.bins.as<uint32_t>(), b.bin_offsets.as<uint32_t>(),
+                         b.bin_counts.as<uint32_t>(), b.headers.as<uint32_t>(), b.events.as<uint32_t>(),
+                         b.err.as<uint32_t>(), s));
+        for (uint32_t lv = ps.level0; lv <= ps.level1; lv++) {
+            const uint32_t items = ps.item_cnt[lv - ps.level0];
+            const bool timed = tm && items && tm->used < RasterTimer::kPairs;
+            if (timed) CK(cudaEventRecord(tm->start[tm->used], s));
+            if (items)
+                CK(launch_raster(p.row_w, p.grid, p.max_depth, streams, b.items.as<WorkItem>() + ps.item_off[lv - ps.level0],
+                                 items, b.counter.as<uint32_t>() + launch++, b.cmds.as<Cmd>(), b.draws.as<DrawRec>(),
+                                 b.paints.as<PaintRec>(), b.grads.as<GradRec>(), b.layers.as<LayerRec>(),
+                                 b.bin_offsets.as<uint32_t>(), b.headers.as<uint32_t>(), b.events.as<uint32_t>(),
+                                 b.stack.as<uint32_t>(), b.hairs.as<HairRec>(), b.hair_spans.as<HairSpan>(),
+                                 b.err.as<uint32_t>(), s));
+            if (timed) CK(cudaEventRecord(tm->stop[tm->used++], s));
+            if (!ps.last) continue;
+            for (const auto &q : sb.patterns) {
+                if (q.level != lv) continue;
+                const float inv[6] = {q.inv.sx, q.inv.ky, q.inv.kx, q.inv.sy, q.inv.tx, q.inv.ty};
+                CK(filter_pattern_shade(b.surf[q.tile].as<uint32_t>(), q.tw, q.th, (float *)b.surf[q.shade].p, q.bx, q.by,
+                                        q.bw, q.bh, inv, q.quality, q.repeat != 0, q.opacity, s));
             }
-            int r = run_filter_job(job, b.surf[job.content].as<uint32_t>(), b.surf[job.result].as<uint32_t>(), scratch,
-                                   s, ferr, &ims);
-            if (scratch.e != cudaSuccess) CK(scratch.e);
-            if (r) { set_error("filter: %s", ferr.c_str()); return r; }
-            if (!ferr.empty()) add_warning("filter: " + ferr + " (layer cleared)");
+            for (const auto &job : sb.jobs) {
+                if (job.level != lv) continue;
+                std::string ferr;
+                std::vector<FeImageSurface> ims;
+                for (uint32_t k = 0; k < job.image_count; k++) {
+                    const FeImageReq &q = sb.fe_images[job.image_first + k];
+                    ims.push_back(FeImageSurface{q.prim, b.surf[q.surface].as<uint32_t>()});
+                }
+                int r = run_filter_job(job, b.surf[job.content].as<uint32_t>(), b.surf[job.result].as<uint32_t>(), scratch,
+                                       s, ferr, &ims);
+                if (scratch.e != cudaSuccess) CK(scratch.e);
+                if (r) { set_error("filter: %s", ferr.c_str()); return r; }
+                if (!ferr.empty()) add_warning("filter: " + ferr + " (layer cleared)");
+            }
         }
     }
     g_stats.draws += ndraws;
@@ -1430,6 +1642,13 @@ int rgpu_test_withhold_window(int enabled) {
 
 int rgpu_test_fail_allocations(uint32_t count) {
     g_fail_allocs.store(count);
+    return RGPU_OK;
+}
+
+int rgpu_test_pass_bytes(uint64_t bytes) {
+    Context &c = ctx();
+    std::lock_guard<std::mutex> lock(c.mu);
+    c.pass_bytes = bytes ? bytes : c.device_bytes / 3;
     return RGPU_OK;
 }
 

@@ -267,12 +267,12 @@ __global__ void k_bin(const EdgeRec *edges, const uint32_t *edge_draw, uint32_t 
             const StreamRec &st = streams[dr.stream];
             const EdgeRec er = edges[e];
             const int32_t y0 = max(er.first_y, dr.start_y), y1 = min(er.first_y + (er.hw >> 8), dr.stop_y - 1);
-            // every row the edge has a (sub)scanline in
-            const int32_t b0 = max((y0 >> dr.shift) + dr.oy, 0), b1 = min((y1 >> dr.shift) + dr.oy, st.out_h - 1);
+            // every row of the pass the edge has a (sub)scanline in
+            const int32_t b0 = max((y0 >> dr.shift) + dr.oy, st.row_lo), b1 = min((y1 >> dr.shift) + dr.oy, st.row_hi - 1);
             if (y1 >= y0 && b1 >= b0) {
                 rows = (uint32_t)(b1 - b0 + 1);
                 step = st.draw_cnt;
-                slot = st.bin_off + (uint32_t)b0 * step + (d - st.draw_off);
+                slot = st.bin_off + (uint32_t)(b0 - st.row_lo) * step + (d - st.draw_off);
             }
         }
     }

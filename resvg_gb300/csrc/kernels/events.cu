@@ -269,8 +269,8 @@ k_events(const StreamRec *streams, uint32_t nstreams, uint32_t ntasks, const Dra
         }
         const StreamRec &st = streams[lo];
         const uint32_t per_row = (st.draw_cnt + 31u) >> 5, t = task - st.task_off;
-        const uint32_t row = t / per_row, d0 = (t - row * per_row) << 5;
-        const uint32_t slot0 = st.bin_off + row * st.draw_cnt + d0, nd = min(32u, st.draw_cnt - d0);
+        const uint32_t r0 = t / per_row, d0 = (t - r0 * per_row) << 5;  // the row, from the pass's first
+        const uint32_t slot0 = st.bin_off + r0 * st.draw_cnt + d0, nd = min(32u, st.draw_cnt - d0);
         uint32_t work = __ballot_sync(0xffffffffu, lane < nd && __ldg(bin_counts + slot0 + lane) != 0u);
         if (lane < nd && !(work >> lane & 1u)) headers[slot0 + lane] = 0u;  // no edges here
         while (work) {
@@ -292,8 +292,8 @@ k_events(const StreamRec *streams, uint32_t nstreams, uint32_t ntasks, const Dra
             r.fill_mask = -1;
             uint32_t boff = 0;
             if (have) {
-                const DrawRec &dr = draws[st.draw_off + (slot - st.bin_off - row * st.draw_cnt)];
-                const int32_t ox = dr.ox, ly = (int32_t)row - dr.oy;
+                const DrawRec &dr = draws[st.draw_off + (slot - st.bin_off - r0 * st.draw_cnt)];
+                const int32_t ox = dr.ox, ly = st.row_lo + (int32_t)r0 - dr.oy;
                 const int32_t xl = max(dr.sect_l, -ox), xr = min(dr.sect_r, st.out_w - ox);
                 const bool aa = dr.shift != 0;
                 boff = __ldg(bin_offsets + slot);

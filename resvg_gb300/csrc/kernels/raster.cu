@@ -519,9 +519,10 @@ k_raster(uint32_t max_row_w, const StreamRec *streams, const WorkItem *items, ui
             return make_int4(L.x, L.y, L.w, L.h);
         };
         int32_t depth = 0;
-        const uint32_t row_slot = st.bin_off + wi.row * st.draw_cnt - st.draw_off;  // + draw: its slot
+        const uint32_t slot0 = st.bin_off + (wi.row - (uint32_t)st.row_lo) * st.draw_cnt;
+        const uint32_t row_slot = slot0 - st.draw_off;  // + draw: its slot
         // the row's lists start here (offsets and slots each fit 32 bits, their sum may not)
-        const uint32_t slot0 = st.bin_off + wi.row * st.draw_cnt, off0 = __ldg(bin_offsets + slot0);
+        const uint32_t off0 = __ldg(bin_offsets + slot0);
         const uint32_t row_loc = off0 + slot0;
         const uint32_t *row_events = events + 4ull * ((unsigned long long)off0 + slot0);
         bool stop = false, failed = false;
