@@ -186,8 +186,10 @@ struct StreamRec {
     uint32_t level;                // dependency level: content streams render before their parents
     uint32_t row_w;                // widest work item, a power of two: 64 .. kRasterMaxRow
     int32_t row_lo, row_hi;        // the rows of one pass (all of them where a submission takes one pass)
+    int32_t x_lo, x_hi;            // its columns, kMaxStrip at most: event pixels count from x_lo
 };
 constexpr uint32_t kRasterMaxRow = 512;
+constexpr int32_t kMaxStrip = 32767;
 
 
 // An anti-aliased hairline stroke (tiny-skia scan/hairline_aa.rs): its line

@@ -442,11 +442,12 @@ void plan_items(Plan &p, Pass &ps, size_t nstreams) {
             const StreamRec &st = recs[si];
             if (st.level != lv) continue;
             // rows wider than row_w in pieces of about equal width
-            const int32_t np = (st.out_w + (int32_t)st.row_w - 1) / (int32_t)st.row_w;
-            const int32_t cw = ((st.out_w + np - 1) / np + 31) & ~31;
+            const int32_t w = st.x_hi - st.x_lo;
+            const int32_t np = (w + (int32_t)st.row_w - 1) / (int32_t)st.row_w;
+            const int32_t cw = ((w + np - 1) / np + 31) & ~31;
             for (int32_t y = st.row_lo; y < st.row_hi; y++)
-                for (int32_t x0 = 0; x0 < st.out_w; x0 += cw)
-                    p.items.push_back(WorkItem{si, (uint32_t)y, x0, std::min(x0 + cw, st.out_w)});
+                for (int32_t x0 = st.x_lo; x0 < st.x_hi; x0 += cw)
+                    p.items.push_back(WorkItem{si, (uint32_t)y, x0, std::min(x0 + cw, st.x_hi)});
         }
         ps.item_off[lv - ps.level0] = (uint32_t)first;
         ps.item_cnt[lv - ps.level0] = (uint32_t)(p.items.size() - first);
@@ -463,7 +464,9 @@ void plan_items(Plan &p, Pass &ps, size_t nstreams) {
 }
 
 // Cuts the submission into passes of at most slot_budget slots (or one row of
-// one stream each) and lists their work items.
+// one stream each) and lists their work items.  Streams wider than events reach
+// (a filter's surface may be five times the canvas) take a pass per kMaxStrip
+// columns.
 int plan_passes(Context &c, Plan &p) {
     SceneBuild &sb = p.sb;
     const size_t ns = sb.streams.size();
@@ -473,7 +476,13 @@ int plan_passes(Context &c, Plan &p) {
     p.passes.clear();
     p.streams.clear();
     uint64_t total = 0;
-    for (const StreamRec &st : sb.streams) total += (uint64_t)st.out_h * st.draw_cnt;
+    bool wide = false;
+    for (StreamRec &st : sb.streams) {
+        total += (uint64_t)st.out_h * st.draw_cnt;
+        wide = wide || st.out_w > kMaxStrip;
+        st.x_lo = 0;
+        st.x_hi = st.out_w;
+    }
     auto open = [&](uint32_t lv0, uint32_t lv1) {
         Pass ps;
         ps.level0 = lv0;
@@ -483,34 +492,43 @@ int plan_passes(Context &c, Plan &p) {
         for (size_t si = 0; si < ns; si++) p.streams[ps.streams + si].row_lo = p.streams[ps.streams + si].row_hi = 0;
         p.passes.push_back(ps);
     };
-    if (total <= budget) {
+    if (total <= budget && !wide) {
         open(0, sb.max_level);
         for (size_t si = 0; si < ns; si++) p.streams[si].row_hi = p.streams[si].out_h;
         plan_items(p, p.passes.back(), ns);
     } else {
         for (uint32_t lv = 0; lv <= sb.max_level; lv++) {
             uint64_t used = 0;
+            bool full = false;  // the pass takes no more
             open(lv, lv);
             for (size_t si = 0; si < ns; si++) {
                 const StreamRec &st = sb.streams[si];
                 if (st.level != lv) continue;
-                for (int32_t y = 0; y < st.out_h;) {
+                for (int32_t x = 0, y = 0; x < st.out_w;) {
+                    const int32_t cols = std::min(kMaxStrip, st.out_w - x);
                     const uint64_t left = budget > used ? budget - used : 0;
                     int64_t rows = st.draw_cnt ? (int64_t)(left / st.draw_cnt) : st.out_h;
-                    if (rows < 1 && used) {  // the pass is full
+                    if (full || (rows < 1 && used)) {
                         p.passes.back().last = false;
                         plan_items(p, p.passes.back(), ns);
                         open(lv, lv);
                         used = 0;
+                        full = false;
                         continue;
                     }
                     rows = std::min<int64_t>(std::max<int64_t>(rows, 1), st.out_h - y);
                     StreamRec &rec = p.streams[p.passes.back().streams + si];
                     rec.row_lo = y;
                     rec.row_hi = y + (int32_t)rows;
+                    rec.x_lo = x;
+                    rec.x_hi = x + cols;
                     used += (uint64_t)rows * st.draw_cnt;
                     y += (int32_t)rows;
-                    if (y < st.out_h) used = std::max(used, budget);  // a stream has one run of rows in a pass
+                    if (y == st.out_h) {
+                        y = 0;
+                        x += cols;
+                    }
+                    full = x < st.out_w;  // a stream has one part in a pass
                 }
             }
             plan_items(p, p.passes.back(), ns);

@@ -31,7 +31,7 @@ constexpr uint32_t kOver = 0xFFFFFFFFu;
 
 // A crossing's sort key: the x of an edge on the sub-scanline relative to the
 // row's first pixel (16.16 sub-columns, below 2^31: anti-aliased rows end below
-// pixel 8192, aliased ones below 32768), and the winding in the lowest bit (-1
+// pixel 8192, aliased ones hold kMaxStrip pixels at most), and the winding in the lowest bit (-1
 // first among equal x, as the reference's sort has it; crossings of equal x and
 // winding commute).  Only crossings inside the row have one: of those left of it
 // the sum of the windings matters alone, `before`, and of those right of it
@@ -69,14 +69,20 @@ __device__ __forceinline__ uint32_t end_entry(int idx) {
     return event_diffs(16 * l - M - c, c - 16 * l);
 }
 
+// A crossing right of pixel 32767.5 rounds, in 32 bits, to -32768: it comes last
+// but its end lies at the row's start (an opening one) or closes a span of no
+// length (a closing one).  Only layers wider than 32767 pixels have such.
+constexpr uint32_t kWide = 3;
+constexpr int32_t kRoundsOver = 0x7FFF8000;
+
 // One sub-scanline of one row of one draw, as its lane sees it.
 struct RowScan {
     const uint32_t *list;  // the draw's binned edges (indices)
     uint32_t nb;           // their number; 0: nothing to draw on this sub-scanline
     int32_t y, base;       // (sub)scanline; the row's first pixel in 16.16 (sub)columns
     uint32_t xmax;         // the row's width in 16.16 (sub)columns
-    uint32_t off;          // the row's first pixel in the stream's row
-    uint32_t kind;         // end_entry's
+    uint32_t off;          // the row's first pixel among the pass's columns
+    uint32_t kind;         // end_entry's; kWide: 2, on a layer wider than 16.16 coordinates reach
     int32_t fill_mask;     // 1 even-odd, -1 non-zero
 };
 
@@ -109,14 +115,19 @@ __device__ __forceinline__ void sort_list(uint32_t *v, uint32_t n) {
 // where contours are clipped.
 __device__ __noinline__ uint32_t crowded(const RowScan &r, const int4 *edges, const uint32_t *ends, uint32_t *v) {
     const uint32_t lane = threadIdx.x & 31u, below = (1u << lane) - 1u;
-    const uint32_t psh = r.kind == 2u ? 0u : 2u, lm = r.kind == 2u ? 0u : 3u;
-    const uint32_t *tab = ends + 16 * r.kind;
+    const uint32_t psh = r.kind >= 2u ? 0u : 2u, lm = r.kind >= 2u ? 0u : 3u;
+    const uint32_t *tab = ends + 16 * min(r.kind, 2u);
     uint32_t n = 0;
     int32_t w = 0;
     for (uint32_t i0 = 0; i0 < r.nb; i0 += 32u) {
         uint32_t key = 0;
-        const bool in = i0 + lane < r.nb &&
-                        crossing_key(__ldg(edges + __ldg(r.list + i0 + lane)), r.y, r.base, r.xmax, &key, &w);
+        bool in = i0 + lane < r.nb &&
+                  crossing_key(__ldg(edges + __ldg(r.list + i0 + lane)), r.y, r.base, r.xmax, &key, &w);
+        // rounds over (key: its distance from the row's start, or 0): last of all
+        if (r.kind == kWide && (key >> 1) >= (uint32_t)kRoundsOver - (uint32_t)r.base && key != 0u) {
+            key = ((r.xmax + 1u) << 1) | (key & 1u);
+            in = true;
+        }
         const uint32_t who = __ballot_sync(0xffffffffu, in);
         if (in) v[1u + n + (uint32_t)__popc(who & below)] = key;
         n += (uint32_t)__popc(who);
@@ -142,8 +153,12 @@ __device__ __noinline__ uint32_t crowded(const RowScan &r, const int4 *edges, co
         upto += w;
         const bool in = ((upto - own) & r.fill_mask) != 0, now = (upto & r.fill_mask) != 0, end = valid && in != now;
         const uint32_t who = __ballot_sync(0xffffffffu, end), opens = __ballot_sync(0xffffffffu, end && now);
-        const uint32_t x = key_sub(key), p = x >> psh, mine = opens & below;
+        const uint32_t mine = opens & below;
+        const bool over = (key >> 1) > r.xmax;  // rounds over
+        uint32_t x = over ? 0u : key_sub(key);
         const uint32_t opened = __shfl_sync(0xffffffffu, x, mine ? 31 - __clz(mine) : 0), from = mine ? opened : left;
+        if (over && in) x = from;
+        const uint32_t p = x >> psh;
         uint32_t t = x & lm;
         if (in) t += ((from & lm) != 0u && (from >> psh) == p) ? 12u : 4u;
         __syncwarp();  // these 32 keys have been read
@@ -204,7 +219,7 @@ __device__ __forceinline__ uint32_t lane_events(uint32_t *col, const RowScan &r,
             n++;
         }
     }
-    const bool over = n > (uint32_t)kMaxSort;
+    const bool over = n > (uint32_t)kMaxSort || r.kind == kWide;
     if (over) n = 0;
     const uint32_t most = __reduce_max_sync(0xffffffffu, n);
     if (most > 16) sort_column<kMaxSort>(keys, n);
@@ -213,8 +228,8 @@ __device__ __forceinline__ uint32_t lane_events(uint32_t *col, const RowScan &r,
     else if (most > 1) sort_column<4>(keys, n);
     // walk: each end of a span overwrites the column from its start (never past
     // the crossings read)
-    const uint32_t psh = r.kind == 2u ? 0u : 2u, lm = r.kind == 2u ? 0u : 3u;
-    const uint32_t *tab = ends + 16 * r.kind;
+    const uint32_t psh = r.kind >= 2u ? 0u : 2u, lm = r.kind >= 2u ? 0u : 3u;
+    const uint32_t *tab = ends + 16 * min(r.kind, 2u);
     uint32_t m = 0, left = 0, f = 0;
     bool in = (w & r.fill_mask) != 0;  // inside a span
     if (in) {  // open at the row's start
@@ -294,7 +309,7 @@ k_events(const StreamRec *streams, uint32_t nstreams, uint32_t ntasks, const Dra
             if (have) {
                 const DrawRec &dr = draws[st.draw_off + (slot - st.bin_off - r0 * st.draw_cnt)];
                 const int32_t ox = dr.ox, ly = st.row_lo + (int32_t)r0 - dr.oy;
-                const int32_t xl = max(dr.sect_l, -ox), xr = min(dr.sect_r, st.out_w - ox);
+                const int32_t xl = max(dr.sect_l, st.x_lo - ox), xr = min(dr.sect_r, st.x_hi - ox);
                 const bool aa = dr.shift != 0;
                 boff = __ldg(bin_offsets + slot);
                 r.y = aa ? ly * 4 + (int32_t)sub : ly;
@@ -302,10 +317,11 @@ k_events(const StreamRec *streams, uint32_t nstreams, uint32_t ntasks, const Dra
                     (aa || sub == 0u)) {
                     r.list = bins + boff;
                     r.nb = __ldg(bin_counts + slot);
-                    r.base = xl << (aa ? 18 : 16);
+                    // past pixel 32767 every crossing lies left of the row
+                    r.base = aa ? xl << 18 : xl > 32767 ? INT32_MAX : xl << 16;
                     r.xmax = (uint32_t)(xr - xl) << (aa ? 18 : 16);
-                    r.off = (uint32_t)(xl + ox);
-                    r.kind = !aa ? 2u : (sub == 3u ? 1u : 0u);
+                    r.off = (uint32_t)(xl + ox - st.x_lo);
+                    r.kind = !aa ? (dr.sect_r > 32767 ? kWide : 2u) : (sub == 3u ? 1u : 0u);
                     r.fill_mask = (dr.flags & DRAW_EVENODD) ? 1 : -1;
                 }
             }
@@ -315,7 +331,7 @@ k_events(const StreamRec *streams, uint32_t nstreams, uint32_t ntasks, const Dra
             const uint32_t overs = __ballot_sync(0xffffffffu, m == kOver);
             if (m == kOver) {
                 first = r.off;
-                last = r.off + (r.xmax >> (r.kind == 2u ? 16 : 18));
+                last = r.off + (r.xmax >> (r.kind >= 2u ? 16 : 18));
             }
             auto scan_of = [&](int src) {
                 RowScan s;

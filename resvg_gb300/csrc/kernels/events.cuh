@@ -33,7 +33,8 @@ namespace dev {
 constexpr uint32_t kManyEvents = 0xFFFu;
 constexpr uint32_t kMaxEvents = (1u << 20) - 1u;
 
-// an event: pixel of the stream's row (15 bits), first difference (9 bits), second (7 bits)
+// an event: pixel of the row from the pass's first column on (15 bits), first
+// difference (9 bits), second (7 bits)
 __host__ __device__ __forceinline__ uint32_t event_diffs(int d0, int d1) {
     return ((uint32_t)(d0 & 0x1FF) << 15) | ((uint32_t)(d1 & 0x7F) << 24);
 }

@@ -427,7 +427,7 @@ __device__ __forceinline__ void hairline(const HairRec &hr, const PaintRec &pr, 
     }
 }
 
-// One draw's coverage of the row piece from x0 on, from its n events (the first
+// One draw's coverage of the row piece from event pixel x0 on, from its n events (the first
 // 32 in shared memory, all of them at `list`): the coverage bytes, and the mask
 // of covered groups (bit g << bits of a group's lanes).
 __device__ __forceinline__ uint32_t make_row(const uint32_t *firsts32, const uint32_t *list, uint32_t n, int32_t x0,
@@ -500,6 +500,7 @@ k_raster(uint32_t max_row_w, const StreamRec *streams, const WorkItem *items, ui
         const int ngroup = (wi.x1 - wi.x0 + 31) >> 5;
         const uint32_t in_piece = 0xFFFFFFFFu >> (32 - (ngroup << bits_sh));
         const int32_t cy = (int32_t)wi.row, x0 = wi.x0, x1 = wi.x1;
+        const int32_t e0 = x0 - st.x_lo, e1 = x1 - st.x_lo;  // the piece among the row's event pixels
         auto out_row = [&]() {
             return reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>((uintptr_t)st.out_ptr) +
                                                 (size_t)cy * st.out_stride) + x0 + lane;
@@ -548,7 +549,7 @@ k_raster(uint32_t max_row_w, const StreamRec *streams, const WorkItem *items, ui
                     const uint32_t slot = row_slot + chunk[lane].a, h = __ldg(headers + slot);
                     n = h >> 20;
                     if (n == dev::kManyEvents) n = h & dev::kMaxEvents;
-                    else if ((int32_t)(h >> 10 & 0x3FFu) > (x1 - 1) >> 5 || (int32_t)(h & 0x3FFu) < x0 >> 5) n = 0;
+                    else if ((int32_t)(h >> 10 & 0x3FFu) > (e1 - 1) >> 5 || (int32_t)(h & 0x3FFu) < e0 >> 5) n = 0;
                     if (n) loc = __ldg(bin_offsets + slot) + slot - row_loc;
                 }
             }
@@ -592,7 +593,7 @@ k_raster(uint32_t max_row_w, const StreamRec *streams, const WorkItem *items, ui
                         load_fill(todo);
                         cp_wait<1>();  // all but the copies just asked for
                         __syncwarp();
-                        groups = make_row(f.events, list, cnt, x0, row_w, diff, cov) & in_piece;
+                        groups = make_row(f.events, list, cnt, e0, row_w, diff, cov) & in_piece;
                     }
                     if (op == CMD_FILL) {
                         if (groups)
