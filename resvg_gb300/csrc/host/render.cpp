@@ -985,9 +985,13 @@ int enqueue_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, RasterTimer *t
         uint32_t tot = 0;
         CK(cudaMemcpyAsync(&tot, totals, 4, cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
+        if (tot == 0xFFFFFFFFu) {  // where the scan's total saturates: edges are numbered in 32 bits
+            set_error("the submission has too many edges: render fewer scenes at a time");
+            return RGPU_ERR_CAPACITY;
+        }
         p.nedges = tot;
-        CK(b.edges.ensure(std::max<uint32_t>(tot, 1) * sizeof(EdgeRec)));
-        CK(b.edge_draw.ensure(std::max<uint32_t>(tot, 1) * 4));
+        CK(b.edges.ensure(std::max<uint64_t>(tot, 1) * sizeof(EdgeRec)));
+        CK(b.edge_draw.ensure(std::max<uint64_t>(tot, 1) * 4));
     }
     uint32_t nedges = p.nedges;
     g_stats.edges += nedges;
