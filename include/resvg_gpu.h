@@ -206,8 +206,9 @@ int rgpu_test_scan(const uint32_t *counts, uint32_t count, uint32_t *offsets, ui
  * 64 scenes or more, else one submission); 1: always one submission; n: n
  * chunks (at most one per scene).  The pixels do not depend on it. */
 int rgpu_set_batch_chunks(uint32_t chunks);
-/* Frees the library's cached device buffers and pinned staging (they grow to
- * the largest render seen and are otherwise kept for reuse). */
+/* Frees the library's cached device buffers (the soft renderer's too) and
+ * pinned staging (they grow to the largest render seen and are otherwise kept
+ * for reuse). */
 int rgpu_trim(void);
 
 /* Where stroke outlines are built when a tree is rendered: 1 (the default) on
@@ -337,7 +338,10 @@ typedef struct rgpu_soft_grads {
     float *points, *colors, *stop_offsets, *stop_colors, *sigma, *opacity;
 } rgpu_soft_grads;
 /* image = composite (premultiplied RGBA, scenes x height x width x 4 floats),
- * blurred = its Gaussian blur.  Synchronous. */
+ * blurred = its Gaussian blur.  Synchronous.  Both passes share scratch of 4
+ * (forward) and 20 (backward) bytes per pixel and path, 1.5 GB at most or one row
+ * of one scene, kept between calls (rgpu_trim releases it); less where memory is
+ * short. */
 int rgpu_soft_forward(const rgpu_soft_batch *batch, float *image, float *blurred, void *stream);
 /* Vector-Jacobian product: given dL/d(blurred) (same layout), writes dL/d of
  * every parameter.  `image` is the forward's composite.  Coverage is

@@ -53,11 +53,16 @@ void set_error(const char *fmt, ...) {
 // Failure-detection test hook: the next this-many device or pinned host
 // allocations of the library fail as if memory were exhausted.
 std::atomic<uint32_t> g_fail_allocs{0};
+}  // namespace
 bool forced_alloc_failure() {
     uint32_t n = g_fail_allocs.load();
     while (n && !g_fail_allocs.compare_exchange_weak(n, n - 1)) {}
     return n != 0;
 }
+namespace soft {
+void release_buffers();  // soft.cu
+}
+namespace {
 
 struct DevBuf {
     void *p = nullptr;
@@ -1704,6 +1709,7 @@ int rgpu_set_batch_chunks(uint32_t chunks) {
 }
 
 int rgpu_trim(void) {
+    soft::release_buffers();
     Context &c = ctx();
     std::lock_guard<std::mutex> lock(c.mu);
     if (c.device < 0) return RGPU_OK;

@@ -40,6 +40,7 @@
 
 namespace rgpu {
 void set_last_error_message(const char *msg);  // render.cpp
+bool forced_alloc_failure();                   // render.cpp
 
 namespace soft {
 namespace {
@@ -869,16 +870,23 @@ struct Buf {
     size_t cap = 0;
     cudaError_t ensure(size_t bytes) {
         if (bytes <= cap) return cudaSuccess;
+        release();
+        cudaError_t e = forced_alloc_failure() ? cudaErrorMemoryAllocation : cudaMalloc(&p, bytes);
+        if (e == cudaSuccess) cap = bytes;
+        else {
+            p = nullptr;
+            cudaGetLastError();  // reported here, not by the next launch
+        }
+        return e;
+    }
+    void release() {
         if (p) cudaFree(p);
         p = nullptr;
         cap = 0;
-        cudaError_t e = cudaMalloc(&p, bytes);
-        if (e == cudaSuccess) cap = bytes;
-        return e;
     }
 };
 std::mutex g_mu;
-Buf g_verts, g_vgrad, g_tmp0, g_tmp1, g_tmp2, g_area, g_col, g_mask, g_flags;
+Buf g_verts, g_vgrad, g_tmp0, g_tmp1, g_tmp2, g_slice, g_flags;
 
 bool valid(const rgpu_soft_batch *b) {
     return b && b->scenes && b->width && b->height && b->paths_per_scene && b->seg_offset && b->points &&
@@ -891,26 +899,31 @@ int fail(cudaError_t e) {
     return RGPU_ERR_CUDA;
 }
 
-// The scratch of a slice of scenes: areas and masks per (row, path), and for the
-// adjoint the colours under each path; at least one row of one scene.  Slices that fit the
-// L2 cache instead (96 MB, one scene of 64 paths on 256^2 pixels each) leave the
-// SMs short of warps: the four kernels took 3.25 ms against 1.84.
+// The scratch of a slice of scenes, one buffer for both passes: areas (4 bytes per
+// pixel and path), for the adjoint the colours under each path (16), and masks;
+// at least one row of one scene.  Slices that fit the L2 cache instead (96 MB, one
+// scene of 64 paths on 256^2 pixels each) leave the SMs short of warps: the four
+// kernels took 3.25 ms against 1.84.  Where memory is short, slices are halved.
 constexpr size_t kSliceBytes = (size_t)1536 << 20;
 cudaError_t make_slice(const rgpu_soft_batch &b, bool adjoint, Slice *sl) {
     sl->ng = (b.width + 31) / 32;
-    const size_t P = b.paths_per_scene, row_px = P * 32 * sl->ng;
-    // rows that fit; warps, one per (row, path) or group of a row, are counted in 32 bits
-    const size_t fit = std::min<size_t>(kSliceBytes / (row_px * (adjoint ? 20 : 4) + P * 4), 0x7FFFFFFFull / (P + sl->ng));
-    sl->rows = (uint32_t)std::min<size_t>(b.height, std::max<size_t>(1, fit));
-    sl->scenes = (uint32_t)std::min<size_t>(b.scenes, std::max<size_t>(1, fit / b.height));
-    const size_t rows = (size_t)sl->scenes * sl->rows;
-    cudaError_t e = g_area.ensure(rows * row_px * sizeof(float));
-    if (e == cudaSuccess && adjoint) e = g_col.ensure(rows * row_px * sizeof(float4));
-    if (e == cudaSuccess) e = g_mask.ensure(rows * P * 4);
-    sl->area = (float *)g_area.p;
-    sl->under = (float4 *)g_col.p;
-    sl->mask = (uint32_t *)g_mask.p;
-    return e;
+    const size_t P = b.paths_per_scene, row_px = P * 32 * sl->ng, row_bytes = row_px * (adjoint ? 20 : 4) + P * 4;
+    for (size_t most = kSliceBytes;;) {
+        // rows that fit; warps, one per (row, path) or group of a row, are counted in 32 bits
+        const size_t fit = std::min<size_t>(most / row_bytes, 0x7FFFFFFFull / (P + sl->ng));
+        sl->rows = (uint32_t)std::min<size_t>(b.height, std::max<size_t>(1, fit));
+        sl->scenes = (uint32_t)std::min<size_t>(b.scenes, std::max<size_t>(1, fit / b.height));
+        const size_t rows = (size_t)sl->scenes * sl->rows;
+        cudaError_t e = g_slice.ensure(rows * row_bytes);
+        if (e == cudaErrorMemoryAllocation && rows > 1) {
+            most = rows * row_bytes / 2;
+            continue;
+        }
+        sl->area = (float *)g_slice.p;
+        sl->under = (float4 *)(sl->area + rows * row_px);
+        sl->mask = (uint32_t *)(sl->area + rows * row_px * (adjoint ? 5 : 1));
+        return e;
+    }
 }
 // CTA size and shared memory of the row kernels for the slice's width
 uint32_t row_warps(const Slice &sl) {
@@ -967,6 +980,13 @@ cudaError_t blur(const float4 *in, float4 *out, float4 *tmp, const rgpu_soft_bat
 }
 
 }  // namespace
+
+// rgpu_trim's share: the work buffers are empty again
+void release_buffers() {
+    std::lock_guard<std::mutex> lock(g_mu);  // every call ends with its stream synchronised
+    for (Buf *b : {&g_verts, &g_vgrad, &g_tmp0, &g_tmp1, &g_tmp2, &g_slice, &g_flags}) b->release();
+}
+
 }  // namespace soft
 }  // namespace rgpu
 

@@ -74,3 +74,58 @@ def test_non_finite_paint_stays_in_its_coverage(gpu, bad, gradient):
     for part in (slice(0, 33), slice(43, w)):
         assert np.isfinite(img[:, :, part]).all() and np.array_equal(img[:, :, part], ref[:, :, part])
     assert not np.isfinite(img[:, :, 33:43]).all()  # the covered ones are spoilt
+
+
+def _failure_hooks():
+    import ctypes as C
+    import resvg_gb300 as R
+    L = R.lib()
+    L.rgpu_test_fail_allocations.argtypes = [C.c_uint32]
+    return L
+
+
+@pytest.mark.parametrize("fail", [1, 3, 6])
+def test_short_memory_makes_smaller_slices(gpu, fail):
+    """Failed allocations of the scratch halve the slices, down to one row; the
+    results do not depend on them (but for the order of the gradients' sums)."""
+    L = _failure_hooks()
+    L.rgpu_trim()
+    # no more lines, but more paths: nothing but the scratch grows
+    few = dict(soft.make_scenes(seed=2, scenes=3, size=96, paths=2, min_segs=64, max_segs=64), height=41)
+    many = dict(soft.make_scenes(seed=3, scenes=3, size=96, paths=32, min_segs=2, max_segs=4), height=41)
+    assert many["seg_offset"][-1] <= few["seg_offset"][-1]
+
+    def step(arrays):
+        sc = soft.Scenes(arrays)
+        image, blurred = soft.forward(sc)
+        return image, blurred, soft.backward(sc, image, blurred)
+
+    ref = step(many)
+    L.rgpu_trim()
+    step(few)
+    L.rgpu_test_fail_allocations(fail)
+    try:
+        got = step(many)
+    finally:
+        L.rgpu_test_fail_allocations(0)
+    assert np.array_equal(got[0].cpu().numpy(), ref[0].cpu().numpy())
+    assert np.array_equal(got[1].cpu().numpy(), ref[1].cpu().numpy())
+    for k in KEYS:
+        a, b = got[2][k].cpu().numpy(), ref[2][k].cpu().numpy()
+        assert np.abs(a - b).max() <= 1e-4 * max(1.0, np.abs(b).max())
+
+
+def test_trim_gives_the_scratch_back(gpu):
+    import torch
+    L = _failure_hooks()
+    a = soft.make_scenes(seed=4, scenes=4, size=512, paths=64, min_segs=2, max_segs=3)
+    sc = soft.Scenes(a)
+    image, blurred = soft.forward(sc)
+    soft.backward(sc, image, blurred)
+    torch.cuda.synchronize()
+    free = torch.cuda.mem_get_info()[0]
+    assert L.rgpu_trim() == 0
+    # 4 x 512^2 pixels x 64 paths x 20 bytes
+    assert torch.cuda.mem_get_info()[0] - free >= 1_300_000_000
+    again, _ = soft.forward(sc)
+    assert torch.equal(again, image)
