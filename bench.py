@@ -411,12 +411,12 @@ def run_batched(args, rank, world):
     stream = torch.cuda.Stream(device=dev)
     torch.cuda.set_stream(stream)
     sh = stream.cuda_stream
-    # autotune the raster decomposition on a stratified sample of the scenes:
-    # band rows per (canvas-width, draw-count) bucket (kept, without effect), then pixels per thread
+    # autotune the raster decomposition (pixels per thread, the width of a row
+    # piece) on a stratified sample of the scenes
     samp = list(range(0, n, max(1, n // 256)))
     t0 = time.perf_counter()
-    table, best_px, tune_ms = BT.autotune_table([trees[i] for i in samp], [ws[i] for i in samp],
-                                                [hs[i] for i in samp], [ptrs[i] for i in samp], reps=2)
+    _, best_px, tune_ms = BT.autotune_table([trees[i] for i in samp], [ws[i] for i in samp],
+                                            [hs[i] for i in samp], [ptrs[i] for i in samp], reps=2)
     tune_s = time.perf_counter() - t0
     t0 = time.perf_counter()
     scene = R.Scene(trees, ident, ws, hs, ptrs)
@@ -512,11 +512,8 @@ def run_batched(args, rank, world):
                    "split": "LPT on side^2 x paths" if world > 1 else "one GPU",
                    "output_mpix": out_px / 1e6, "draws": info["draws"], "edges": info["edges"],
                    "binned_edges": info["binned_edges"], "work_items": info["work_items"],
-                   "tuning": {"table": [list(e) for e in table], "pixels_per_thread": best_px,
-                              "autotune_ms_on_sample": min(min(v.values()) for v in tune_ms.values()),
-                              "autotune_s": tune_s,
-                              "buckets": "width <= %s x draws <= %s" % (list(BT.WIDTH_BUCKETS),
-                                                                        list(BT.DRAW_BUCKETS))},
+                   "tuning": {"pixels_per_thread": best_px,
+                              "autotune_ms_on_sample": min(tune_ms["global"].values()), "autotune_s": tune_s},
                    "prepare_s": prep_s, "stroke": stroke, "l2": "outputs %.1f GB > L2 (129 MB)" % (total / 1e9),
                    "graph_replay": True},
         "mpix_s": value * out_px / n / 1e6 if n else 0.0,
@@ -681,8 +678,8 @@ def run_plain(args, rank, world):
     tree = R.Tree.generate(args.config, seed=SEED, index=rank, scale=args.scale)
     w, h = (int(v) for v in tree.size)
     surface = torch.zeros((h, w, 4), dtype=torch.uint8, device=dev)
-    # the product's autotuner (rgpu_autotune) picks band rows and pixels per
-    # thread for this scene, on a copy of the tree: the timed tree's own first
+    # the product's autotuner (rgpu_autotune) picks pixels per thread for this
+    # scene, on a copy of the tree: the timed tree's own first
     # render is the one that strokes its paths
     t0 = time.perf_counter()
     tune_tree = R.Tree.generate(args.config, seed=SEED, index=rank, scale=args.scale)

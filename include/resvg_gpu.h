@@ -170,7 +170,8 @@ int rgpu_get_tuning_table(rgpu_tuning_entry *entries, uint32_t capacity, uint32_
 /* Autotuner (no counterpart in the reference): prepares the given scenes once
  * per candidate tuning, times `reps` graph replays of each with CUDA events,
  * keeps the fastest as the current tuning and returns it (and its ms per
- * render).  Candidates that fail are skipped. */
+ * render).  Candidates that fail are skipped, and those that differ from an
+ * earlier one in band rows alone are that one. */
 int rgpu_autotune(const resvg_render_tree *const *trees, const resvg_transform *transforms, uint32_t count,
                   const uint32_t *widths, const uint32_t *heights, uint8_t *const *device_pixmaps,
                   const uint32_t *strides, const rgpu_tuning *candidates, uint32_t candidate_count, uint32_t reps,

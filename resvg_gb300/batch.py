@@ -15,11 +15,11 @@ import numpy as np
 
 # (band rows, pixels per thread) the autotuner searches.  Work items are single
 # rows, so band rows make no difference; pixels per thread set the width of a row
-# piece (32 times as many pixels).
-TUNING_CANDIDATES = [(0, 8), (0, 16), (1, 4), (2, 4), (4, 4), (2, 8), (4, 8), (8, 8), (4, 16), (8, 16)]
+# piece (32 times as many pixels), 0 leaves it to the rule by the level's rows.
+TUNING_CANDIDATES = [(0, 0), (0, 4), (0, 8), (0, 16)]
 
 # Buckets of the tuning table: stream width (canvas side) and draws (fills and
-# strokes), upper bounds; the band heights tried per bucket.
+# strokes), upper bounds; the band heights an entry may hold.
 WIDTH_BUCKETS = (128, 256, 512, 1024, 32767)
 DRAW_BUCKETS = (64, 256, 1024, 1 << 30)
 BAND_CANDIDATES = (1, 2, 4, 8)
@@ -57,66 +57,30 @@ def _time_scene(R, torch, trees, widths, heights, ptrs, stream, reps):
 
 def autotune_table(trees, widths, heights, device_ptrs, reps: int = 2, min_share: float = 0.05,
                    min_gain: float = 0.01):
-    """The batched form's autotuner; every timing renders the whole sample as
-    one prepared batch, so each choice is judged where it runs.
-
-    1. (band rows, pixels per thread) over TUNING_CANDIDATES, one value for
-       every stream: the best pair is the starting point.
-    2. Scenes are grouped by (canvas-width bucket, draw-count bucket); for
-       every bucket holding at least `min_share` of the sample's estimated
-       cost (side^2 x draws), heaviest first, the other band heights are tried
-       for that bucket alone and kept when the batch gets faster by more than
-       `min_gain`.
-    Installs the table and the pixels per thread, and returns (table, pixels
-    per thread, {"global": {candidate: ms}, bucket: {band rows: ms}})."""
+    """The batched form's autotuner: renders the whole sample as one prepared
+    batch under every one of TUNING_CANDIDATES and installs the fastest.  The
+    table's band rows choose nothing (work items are single rows), so its
+    entries are left automatic, and `min_share` and `min_gain` of the earlier
+    search per bucket have no effect.  Returns (table, pixels per thread,
+    {"global": {candidate: ms}})."""
     import torch
     import resvg_gb300 as R
     stream = torch.cuda.Stream()
     saved = R.get_tuning()
-    args = (trees, widths, heights, device_ptrs, stream, reps)
     timings = {"global": {}}
     try:
         R.set_tuning_table([])
         for b, px in TUNING_CANDIDATES:
             R.set_tuning(b, px)
-            timings["global"][(b, px)] = _time_scene(R, torch, *args)
-        (b0, px0), best = min(timings["global"].items(), key=lambda kv: kv[1])
-        cost = {}
-        for i, t in enumerate(trees):
-            d = scene_draws(t)
-            key = bucket_of(widths[i], d)
-            cost[key] = cost.get(key, 0.0) + scene_cost(widths[i], heights[i], d)
-        total = sum(cost.values()) or 1.0
-        # a table entry for every bucket, starting from the global band height
-        # (band rows 0 keeps the per-stream rule of that candidate)
-        table = {(wb, db): b0 for wb in WIDTH_BUCKETS for db in DRAW_BUCKETS}
-
-        def install():
-            R.set_tuning_table([(wb, db, table[(wb, db)]) for wb in WIDTH_BUCKETS for db in DRAW_BUCKETS])
-        R.set_tuning(0, px0)
-        install()
-        for key in sorted(cost, key=cost.get, reverse=True):
-            if cost[key] / total < min_share:
-                break
-            res = {table[key]: best}
-            for b in BAND_CANDIDATES:
-                if b == table[key]:
-                    continue
-                keep = table[key]
-                table[key] = b
-                install()
-                res[b] = _time_scene(R, torch, *args)
-                if res[b] < best * (1.0 - min_gain):
-                    best = res[b]
-                else:
-                    table[key] = keep
-            install()
-            timings[key] = res
-        entries = [(wb, db, table[(wb, db)]) for wb in WIDTH_BUCKETS for db in DRAW_BUCKETS]
+            timings["global"][(b, px)] = _time_scene(R, torch, trees, widths, heights, device_ptrs, stream, reps)
+        (_, best_px), _ = min(timings["global"].items(), key=lambda kv: kv[1])
+        entries = [(wb, db, 0) for wb in WIDTH_BUCKETS for db in DRAW_BUCKETS]
+        R.set_tuning(0, best_px)
+        R.set_tuning_table(entries)
     except Exception:
         R.set_tuning(*saved)
         raise
-    return entries, px0, timings
+    return entries, best_px, timings
 
 
 def scene_cost(width: float, height: float, paths: int) -> float:

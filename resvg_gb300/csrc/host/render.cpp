@@ -1618,8 +1618,14 @@ int rgpu_autotune(const resvg_render_tree *const *trees, const resvg_transform *
     if (cudaEventCreate(&e1) != cudaSuccess) { cudaEventDestroy(e0); set_error("event"); return RGPU_ERR_CUDA; }
     float best_t = 0.0f;
     int best_i = -1, last_err = RGPU_OK;
+    std::vector<bool> tried(ncand);
     for (uint32_t i = 0; i < ncand; i++) {
         if (rgpu_set_tuning(&candidates[i]) != RGPU_OK) continue;
+        // band rows choose nothing: only the first candidate of each row width is timed
+        bool timed = false;
+        for (uint32_t k = 0; k < i; k++)
+            timed = timed || (tried[k] && candidates[k].pixels_per_thread == candidates[i].pixels_per_thread);
+        if (timed) continue;
         rgpu_scene *sc = nullptr;
         int r = rgpu_scene_prepare(trees, transforms, count, widths, heights, device_pixmaps, strides, &sc);
         // first render sizes the buffers, the second captures the graph
@@ -1637,6 +1643,7 @@ int rgpu_autotune(const resvg_render_tree *const *trees, const resvg_transform *
         }
         if (sc) rgpu_scene_free(sc);
         if (r != RGPU_OK) { last_err = r; continue; }
+        tried[i] = true;
         if (best_i < 0 || ms < best_t) { best_t = ms; best_i = (int)i; }
     }
     cudaEventDestroy(e0);

@@ -249,3 +249,17 @@ def test_tuning_table_autotuner_renders_exactly(tuning_case):
     finally:
         R.set_tuning_table([])
         R.set_tuning(*saved)
+
+
+def test_autotuner_times_a_row_width_once(tuning_case):
+    """Candidates that differ in band rows alone are the same rendering: the first
+    of each row width stands for the rest, whatever the timings' noise."""
+    trees, _ = tuning_case
+    saved = R.get_tuning()
+    try:
+        db = _DeviceBatch(trees)
+        cands = [(8, 16), (0, 16), (4, 16), (2, 16), (1, 16)]
+        best, ms = R.autotune(trees, [IDENT] * len(trees), db.ws, db.hs, db.ptrs, cands, reps=1)
+        assert tuple(best) == (8, 16) and ms > 0
+    finally:
+        R.set_tuning(*saved)
