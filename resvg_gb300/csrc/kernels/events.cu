@@ -40,16 +40,13 @@ constexpr uint32_t kOver = 0xFFFFFFFFu;
 __device__ __forceinline__ bool crossing_key(const int4 &e, int32_t y, int32_t base, uint32_t xmax, uint32_t *key,
                                              int32_t *before) {
     const int32_t dy = y - e.z;
-    if ((uint32_t)dy > (uint32_t)(e.w >> 8)) return false;
+    const bool hit = (uint32_t)dy <= (uint32_t)(e.w >> 8);
     const int32_t X = (int32_t)((uint32_t)e.x + (uint32_t)dy * (uint32_t)e.y);
-    const uint32_t up = (e.w & 0x80) ? 0u : 1u;
-    if (X <= base) {
-        *before += (int32_t)(up << 1) - 1;
-        return false;
-    }
-    const uint32_t d = (uint32_t)X - (uint32_t)base;
-    *key = (d << 1) | up;
-    return d < xmax;
+    const uint32_t up = (e.w & 0x80) ? 0u : 1u, d = (uint32_t)X - (uint32_t)base;
+    const bool left = X <= base;
+    *before += hit && left ? (int32_t)(up << 1) - 1 : 0;
+    *key = hit && !left ? (d << 1) | up : 0u;
+    return hit && !left && d < xmax;
 }
 // the key's x rounded to a sub-column: ((key >> 1) + 0x8000) >> 16
 __device__ __forceinline__ uint32_t key_sub(uint32_t key) { return (key + 0x10000u) >> 17; }

@@ -49,7 +49,7 @@ struct FillSlot {
 
 struct WarpShared {
     unsigned long long mb;           // mbarrier of the command copies
-    unsigned long long _pad;
+    int32_t first, _pad;             // the piece's first pixel among the row's event pixels (no register held)
     Cmd chunk[2][kChunk];            // the current commands and the next
     uint32_t rect[kMaxDepth];        // layer-stack layers by depth
     PaintRec hair_paint;             // the current hairline's paint
@@ -500,7 +500,7 @@ k_raster(uint32_t max_row_w, const StreamRec *streams, const WorkItem *items, ui
         const int ngroup = (wi.x1 - wi.x0 + 31) >> 5;
         const uint32_t in_piece = 0xFFFFFFFFu >> (32 - (ngroup << bits_sh));
         const int32_t cy = (int32_t)wi.row, x0 = wi.x0, x1 = wi.x1;
-        const int32_t e0 = x0 - st.x_lo, e1 = x1 - st.x_lo;  // the piece among the row's event pixels
+        if (lane == 0) ws.first = x0 - st.x_lo;
         auto out_row = [&]() {
             return reinterpret_cast<uint32_t *>(reinterpret_cast<uint8_t *>((uintptr_t)st.out_ptr) +
                                                 (size_t)cy * st.out_stride) + x0 + lane;
@@ -549,7 +549,7 @@ k_raster(uint32_t max_row_w, const StreamRec *streams, const WorkItem *items, ui
                     const uint32_t slot = row_slot + chunk[lane].a, h = __ldg(headers + slot);
                     n = h >> 20;
                     if (n == dev::kManyEvents) n = h & dev::kMaxEvents;
-                    else if ((int32_t)(h >> 10 & 0x3FFu) > (e1 - 1) >> 5 || (int32_t)(h & 0x3FFu) < e0 >> 5) n = 0;
+                    else if ((int32_t)(h >> 10 & 0x3FFu) > (ws.first + (x1 - x0) - 1) >> 5 || (int32_t)(h & 0x3FFu) < ws.first >> 5) n = 0;
                     if (n) loc = __ldg(bin_offsets + slot) + slot - row_loc;
                 }
             }
@@ -593,7 +593,7 @@ k_raster(uint32_t max_row_w, const StreamRec *streams, const WorkItem *items, ui
                         load_fill(todo);
                         cp_wait<1>();  // all but the copies just asked for
                         __syncwarp();
-                        groups = make_row(f.events, list, cnt, e0, row_w, diff, cov) & in_piece;
+                        groups = make_row(f.events, list, cnt, ws.first, row_w, diff, cov) & in_piece;
                     }
                     if (op == CMD_FILL) {
                         if (groups)

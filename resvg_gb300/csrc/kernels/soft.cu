@@ -359,12 +359,12 @@ k_area(rgpu_soft_batch B, Slice sl, const float2 *verts, uint32_t *overflow) {
 // colour whatever the paint (an infinite one would make it NaN)
 __device__ __forceinline__ void composite(float4 &C, float A, const PaintOut &po) {
     const float c = fminf(fabsf(A), 1.0f);
-    if (c == 0.0f) return;
+    const bool on = c != 0.0f;  // selects: a branch per group took 5% more of a small step
     const float ca = c * po.a, keep = 1.0f - ca;
-    C.x = c * (po.r * po.a) + keep * C.x;
-    C.y = c * (po.g * po.a) + keep * C.y;
-    C.z = c * (po.b * po.a) + keep * C.z;
-    C.w = ca + keep * C.w;
+    C.x = on ? c * (po.r * po.a) + keep * C.x : C.x;
+    C.y = on ? c * (po.g * po.a) + keep * C.y : C.y;
+    C.z = on ? c * (po.b * po.a) + keep * C.z : C.z;
+    C.w = on ? ca + keep * C.w : C.w;
 }
 
 // the warp's row and groups: G neighbouring groups of one row
