@@ -1012,9 +1012,6 @@ int enqueue_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, RasterTimer *t
         p.sized = true;
     }
     CK(cudaMemsetAsync(b.err.p, 0, 4, s));
-    CK(cudaMemsetAsync(b.counter.p, 0, 4 * std::max<size_t>(p.raster_launches, 1), s));
-    for (const auto &st : sb.streams)
-        if (st.surface >= 0) CK(cudaMemsetAsync(b.surf[st.surface].p, 0, (size_t)st.out_w * st.out_h * 4, s));
     BufScratch scratch(b);
     if (tm) {
         CK(tm->ensure());
@@ -1035,6 +1032,11 @@ int enqueue_plan(Context &c, Buffers &b, Plan &p, cudaStream_t s, RasterTimer *t
                          b.edges.as<EdgeRec>(), b.bins.as<uint32_t>(), b.bin_offsets.as<uint32_t>(),
                          b.bin_counts.as<uint32_t>(), b.headers.as<uint32_t>(), b.events.as<uint32_t>(),
                          b.err.as<uint32_t>(), s));
+        if (&ps == &p.passes.front()) {
+            CK(cudaMemsetAsync(b.counter.p, 0, 4 * std::max<size_t>(p.raster_launches, 1), s));
+            for (const auto &st : sb.streams)
+                if (st.surface >= 0) CK(cudaMemsetAsync(b.surf[st.surface].p, 0, (size_t)st.out_w * st.out_h * 4, s));
+        }
         for (uint32_t lv = ps.level0; lv <= ps.level1; lv++) {
             const uint32_t items = ps.item_cnt[lv - ps.level0];
             const bool timed = tm && items && tm->used < RasterTimer::kPairs;
