@@ -258,6 +258,7 @@ struct Context {
     int sms = 0;
     uint64_t pass_bytes = 0;     // working memory of a pass, at most
     uint64_t device_bytes = 0;
+    int raster_blocks[4] = {};   // k_raster's CTAs per SM by row width (64 .. 512), once asked for
     cudaStream_t stream = nullptr;
     RasterTimer timer;
     Buffers buf;
@@ -345,9 +346,9 @@ int upload(HostBuf &staging, DevBuf &d, const std::vector<T> &v, size_t &stage_o
 // them leave the SMs idle: 512 pixels against 128 measured 8.8 against 11.4 ms
 // on 1024^2 pixels (2048 items), 0.55 against 0.50 ms on 512^2 (512 items) and
 // 1.01 against 0.82 ms on 301 x 333.  1024 pixels were never the fastest.
-constexpr uint64_t kMinItems = 1536;
-uint32_t pick_row_w(const SceneBuild &sb, uint32_t level, const Tuning &tu) {
+uint32_t pick_row_w(const SceneBuild &sb, uint32_t level, const Tuning &tu, int sms) {
     if (tu.px) return 32 * tu.px;
+    const uint64_t min_items = 10ull * (uint64_t)sms;
     uint32_t w = 512;
     for (; w > 64; w /= 2) {
         uint64_t n = 0;
@@ -357,7 +358,7 @@ uint32_t pick_row_w(const SceneBuild &sb, uint32_t level, const Tuning &tu) {
                 n += (uint64_t)st.out_h * ((st.out_w + w - 1) / w);
                 wide = wide || (uint32_t)st.out_w > w / 2;
             }
-        if (n >= kMinItems && wide) break;
+        if (n >= min_items && wide) break;
     }
     return w;
 }
@@ -550,8 +551,9 @@ int plan_passes(Context &c, Plan &p) {
         }
     }
     if (p.nbins > 0xF0000000ull) { set_error("a row holds too many draws"); return RGPU_ERR_CAPACITY; }
-    uint32_t per_sm = (uint32_t)raster_max_blocks_per_sm(p.row_w);
-    p.grid = std::max<uint32_t>(1, std::min<uint32_t>(most, (uint32_t)c.sms * per_sm));
+    int &per_sm = c.raster_blocks[p.row_w <= 64 ? 0 : p.row_w <= 128 ? 1 : p.row_w <= 256 ? 2 : 3];
+    if (!per_sm) per_sm = raster_max_blocks_per_sm(p.row_w);
+    p.grid = std::max<uint32_t>(1, std::min<uint32_t>(most, (uint32_t)(c.sms * per_sm)));
     return RGPU_OK;
 }
 
@@ -623,7 +625,7 @@ int plan_scene(Context &c, Plan &p) {
     p.row_w = 64;
     p.max_depth = 1;
     std::vector<uint32_t> level_w(sb.max_level + 1);
-    for (uint32_t lv = 0; lv <= sb.max_level; lv++) level_w[lv] = pick_row_w(sb, lv, c.tuning);
+    for (uint32_t lv = 0; lv <= sb.max_level; lv++) level_w[lv] = pick_row_w(sb, lv, c.tuning, c.sms);
     for (StreamRec &st : sb.streams) {
         st.row_w = level_w[st.level];
         p.row_w = std::max(p.row_w, st.row_w);

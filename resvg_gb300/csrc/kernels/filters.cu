@@ -23,6 +23,17 @@
 namespace rgpu {
 namespace {
 
+// SMs of the current device (a grid that walks its work needs no more CTAs than fit)
+unsigned sm_count() {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || n < 1) {
+        cudaGetLastError();
+        n = 1;
+    }
+    return (unsigned)n;
+}
+
 __constant__ __align__(16) uint8_t c_srgb_to_linear[256];
 __constant__ __align__(16) uint8_t c_linear_to_srgb[256];
 
@@ -930,7 +941,7 @@ cudaError_t filter_iir_blur(uint32_t *img, double *buf, int w, int h, double sx,
         return iir_blur_fast(img, reinterpret_cast<float *>(buf), reinterpret_cast<float *>(buf) + 4 * n, w, h, dx,
                              dy, sx > 0.0, sy > 0.0, post, s);
     // buf holds four planes of n doubles
-    k_iir_load4<<<std::min(nblk(n, 256), 1216u), 256, 0, s>>>(img, buf, n);  // 8 CTAs on each of 152 SMs
+    k_iir_load4<<<std::min(nblk(n, 256), 8u * sm_count()), 256, 0, s>>>(img, buf, n);  // 8 CTAs on each SM
     if (sx > 0.0) k_iir_rows4<<<nblk((size_t)4 * h, 64), 64, 0, s>>>(buf, w, h, dx, steps);
     if (sy > 0.0) k_iir_cols4<<<nblk((size_t)4 * w, 64), 64, 0, s>>>(buf, w, h, dy, steps);
     k_iir_store4<<<nblk(n, 256), 256, 0, s>>>(img, buf, n, post);
