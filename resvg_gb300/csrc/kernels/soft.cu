@@ -194,8 +194,8 @@ __device__ __forceinline__ uint32_t path_nverts(const rgpu_soft_batch &B, uint32
 // the adjoint later dL/dA), the colours under the path, and a mask of the
 // groups the path covers.  The scenes, and the rows of a scene that is too large
 // by itself, are taken in slices of bounded scratch.
-// On 16 scenes of 64 paths on 256^2 pixels: areas 0.32 ms, composite 0.16 ms, its
-// reverse 0.72 ms, line gradients 0.32 ms.  (One CTA per row doing all of it in
+// On 16 scenes of 64 paths on 256^2 pixels: areas 0.32 ms, composite 0.15 ms, its
+// reverse 0.56 ms, line gradients 0.32 ms.  (One CTA per row doing all of it in
 // turn, with a block barrier for every step of every path, took 1.10 ms forward
 // and 5.42 ms for the adjoint.)
 struct Slice {
@@ -384,35 +384,24 @@ struct Strip {
     }
 };
 
-// ---- forward composite
-template <int G>
+// ---- forward composite: one group per warp (see wide_strips)
 __global__ void __launch_bounds__(128) k_composite(rgpu_soft_batch B, Slice sl, float4 *image) {
-    const Strip<G> st(B, sl);
+    const Strip<1> st(B, sl);
     if (!st.ok) return;
-    const int lane = threadIdx.x & 31, W = (int)B.width;
+    const int lane = threadIdx.x & 31, W = (int)B.width, x = (int)(32 * st.g0) + lane;
     const uint32_t P = B.paths_per_scene;
-    float4 C[G];
-#pragma unroll
-    for (int k = 0; k < G; k++) C[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+    float4 C = make_float4(0.f, 0.f, 0.f, 0.f);
     const size_t r = st.r;
     for (uint32_t p0 = 0; p0 < P; p0 += 32) {
         // 32 paths' masks at a time; those without coverage here are skipped
-        const uint32_t m = p0 + (uint32_t)lane < P ? (sl.mask[r * P + p0 + (uint32_t)lane] >> st.g0) & ((1u << G) - 1u) : 0u;
-        for (uint32_t todo = __ballot_sync(0xffffffffu, m != 0u); todo; todo &= todo - 1u) {
-            const int l = __ffs(todo) - 1;
-            const uint32_t p = p0 + (uint32_t)l, mp = __shfl_sync(0xffffffffu, m, l), j = (sl.s0 + st.sc) * P + p;
-            const float *area = sl.area + (r * P + p) * (32 * sl.ng) + 32 * st.g0 + (uint32_t)lane;
-#pragma unroll
-            for (int k = 0; k < G; k++)
-                if (mp >> k & 1u)
-                    composite(C[k], area[32 * k], eval_paint(B, j, (float)(32 * (st.g0 + k) + lane) + 0.5f, (float)st.row + 0.5f));
+        const bool m = p0 + (uint32_t)lane < P && (sl.mask[r * P + p0 + (uint32_t)lane] >> st.g0 & 1u) != 0u;
+        for (uint32_t todo = __ballot_sync(0xffffffffu, m); todo; todo &= todo - 1u) {
+            const uint32_t p = p0 + (uint32_t)__ffs(todo) - 1u, j = (sl.s0 + st.sc) * P + p;
+            composite(C, sl.area[(r * P + p) * (32 * sl.ng) + 32 * st.g0 + (uint32_t)lane],
+                      eval_paint(B, j, (float)x + 0.5f, (float)st.row + 0.5f));
         }
     }
-#pragma unroll
-    for (int k = 0; k < G; k++) {
-        const int x = (int)(32 * (st.g0 + k)) + lane;
-        if (x < W) image[((size_t)(sl.s0 + st.sc) * B.height + st.row) * W + x] = C[k];
-    }
+    if (x < W) image[((size_t)(sl.s0 + st.sc) * B.height + st.row) * W + x] = C;
 }
 
 // ---- flattening: one thread per (path, vertex)
@@ -931,12 +920,18 @@ uint32_t row_warps(const Slice &sl) {
 }
 uint32_t blocks(uint64_t n, uint32_t per) { return (uint32_t)((n + per - 1) / per); }
 
-// Groups per warp of the composite kernels: two where there are plenty (a path's
-// paint gradients are reduced once per warp), one where a warp, a chain over the
-// paths, would leave the SMs too little to do.  Reverse composite of 16 scenes of
-// 256^2 pixels: two 0.72 ms, four 0.77, eight 1.12.
+// Groups per warp of the reverse composite.  Every warp adds its share of a path's
+// paint gradients to the same words, so where many groups of a scene do that and
+// a warp's chain over the paths is short, two groups per warp halve the adds.  One
+// / two groups, us: 500^2 pixels x 4 paths 15.8 / 11.9, x 64 paths 185 / 188; 16
+// scenes of 256 x 512 x 16 385 / 309; but 16 of 256^2 x 64 558 / 757, 1 of 256^2 x 4
+// 9.5 / 11.9.  The lines lie at 192 groups per path and 6,000 in all (640^2 x 64, 200
+// per path, 0.91 .. 1.01; 256^2 x 16, 128 per path, 0.91 .. 1.39; 256 x 512 x 4, 4,096
+// in all, 1.05; 500^2 x 4, 8,000, 0.75).  The forward composite adds nothing up: one
+// group is never slower there by more than 7%, and up to a third faster.
 bool wide_strips(const rgpu_soft_batch &b, const Slice &sl) {
-    return sl.ng >= 2 && (uint64_t)sl.scenes * sl.rows * sl.ng >= 8192;
+    const uint64_t per_scene = (uint64_t)b.height * sl.ng, all = (uint64_t)sl.scenes * sl.rows * sl.ng;
+    return sl.ng >= 2 && per_scene >= 192ull * b.paths_per_scene && all >= 6000;
 }
 template <class F>
 void with_groups(bool wide, F f) {
@@ -1010,11 +1005,7 @@ extern "C" int rgpu_soft_forward(const rgpu_soft_batch *b, float *image, float *
     cudaMemsetAsync(g_flags.p, 0, 16, s);
     each_slice(*b, slice, [&](const Slice &sl) {
         launch_area(*b, sl, s);
-        with_groups(wide_strips(*b, sl), [&](auto G) {
-            constexpr int kG = decltype(G)::value;
-            const uint64_t warps = (uint64_t)sl.scenes * sl.rows * ((sl.ng + kG - 1) / kG);
-            k_composite<kG><<<blocks(warps, 4), 128, 0, s>>>(*b, sl, (float4 *)image);
-        });
+        k_composite<<<blocks((uint64_t)sl.scenes * sl.rows * sl.ng, 4), 128, 0, s>>>(*b, sl, (float4 *)image);
     });
     e = blur((const float4 *)image, (float4 *)blurred, (float4 *)g_tmp0.p, *b, s);
     uint32_t ovf = 0;
