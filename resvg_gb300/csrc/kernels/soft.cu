@@ -835,21 +835,49 @@ k_lines(rgpu_soft_batch B, Slice sl, const float2 *verts, float2 *vgrad) {
     });
 }
 
-__global__ void k_mse(const float *a, const float *b, size_t n, float scale, float *loss, float *grad) {
-    __shared__ float red[32];
+// The loss: every block's share in 64 bits, and the sum of the shares, in their
+// order, by the block that finishes last (`done` counts them and is zero again
+// after it).  Added up in 32 bits in the order of arrival it differed by 2e-6 from
+// run to run.
+constexpr int kMseBlocks = 1024, kMseThreads = 256;
+struct MseScratch {
+    double share[kMseBlocks];
+    uint32_t done;
+};
+__device__ __forceinline__ double block_sum(double v, double *red) {
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    v = 0.0;
+    for (int i = 0; i < kMseThreads / 32; i++) v += red[i];
+    return v;
+}
+__global__ void __launch_bounds__(kMseThreads)
+k_mse(const float *a, const float *b, size_t n, float scale, float *loss, float *grad, MseScratch *scratch) {
+    __shared__ double red[kMseThreads / 32];
+    __shared__ bool last;
     float sum = 0.0f;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const float d = a[i] - b[i];
         sum += d * d;
         if (grad) grad[i] = 2.0f * d * scale;
     }
-    sum = warp_sum(sum);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = sum;
-    __syncthreads();
+    const double share = block_sum((double)sum, red);
     if (threadIdx.x == 0) {
-        float t = 0.0f;
-        for (int i = 0; i < (int)(blockDim.x / 32); i++) t += red[i];
-        atomicAdd(loss, t * scale);
+        scratch->share[blockIdx.x] = share;
+        __threadfence();
+        last = atomicAdd(&scratch->done, 1u) == gridDim.x - 1u;
+    }
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    double all = 0.0;
+    for (int i = (int)threadIdx.x; i < kMseBlocks; i += kMseThreads) all += __ldcg(&scratch->share[i]);
+    all = block_sum(all, red);
+    if (threadIdx.x == 0) {
+        *loss = (float)(all * (double)scale);
+        scratch->done = 0u;
     }
 }
 
@@ -875,7 +903,7 @@ struct Buf {
     }
 };
 std::mutex g_mu;
-Buf g_verts, g_vgrad, g_tmp0, g_tmp1, g_tmp2, g_slice, g_flags;
+Buf g_verts, g_vgrad, g_tmp0, g_tmp1, g_tmp2, g_slice, g_flags, g_mse;
 
 bool valid(const rgpu_soft_batch *b) {
     return b && b->scenes && b->width && b->height && b->paths_per_scene && b->seg_offset && b->points &&
@@ -925,13 +953,14 @@ uint32_t blocks(uint64_t n, uint32_t per) { return (uint32_t)((n + per - 1) / pe
 // a warp's chain over the paths is short, two groups per warp halve the adds.  One
 // / two groups, us: 500^2 pixels x 4 paths 15.8 / 11.9, x 64 paths 185 / 188; 16
 // scenes of 256 x 512 x 16 385 / 309; but 16 of 256^2 x 64 558 / 757, 1 of 256^2 x 4
-// 9.5 / 11.9.  The lines lie at 192 groups per path and 6,000 in all (640^2 x 64, 200
-// per path, 0.91 .. 1.01; 256^2 x 16, 128 per path, 0.91 .. 1.39; 256 x 512 x 4, 4,096
+// 9.5 / 11.9.  The lines lie at 160 groups per path and 6,000 in all (640^2 x 64, 200
+// per path, 0.91 .. 1.01; 13 of 117 x 544 x 12, 181 per path, the step 0.98; 256^2 x 16,
+// 128 per path, 0.91 .. 1.39; 256 x 512 x 4, 4,096
 // in all, 1.05; 500^2 x 4, 8,000, 0.75).  The forward composite adds nothing up: one
 // group is never slower there by more than 7%, and up to a third faster.
 bool wide_strips(const rgpu_soft_batch &b, const Slice &sl) {
     const uint64_t per_scene = (uint64_t)b.height * sl.ng, all = (uint64_t)sl.scenes * sl.rows * sl.ng;
-    return sl.ng >= 2 && per_scene >= 192ull * b.paths_per_scene && all >= 6000;
+    return sl.ng >= 2 && per_scene >= 160ull * b.paths_per_scene && all >= 6000;
 }
 template <class F>
 void with_groups(bool wide, F f) {
@@ -979,7 +1008,7 @@ cudaError_t blur(const float4 *in, float4 *out, float4 *tmp, const rgpu_soft_bat
 // rgpu_trim's share: the work buffers are empty again
 void release_buffers() {
     std::lock_guard<std::mutex> lock(g_mu);  // every call ends with its stream synchronised
-    for (Buf *b : {&g_verts, &g_vgrad, &g_tmp0, &g_tmp1, &g_tmp2, &g_slice, &g_flags}) b->release();
+    for (Buf *b : {&g_verts, &g_vgrad, &g_tmp0, &g_tmp1, &g_tmp2, &g_slice, &g_flags, &g_mse}) b->release();
 }
 
 }  // namespace soft
@@ -1093,10 +1122,17 @@ extern "C" int rgpu_soft_mse(const float *blurred, const float *target, size_t c
         rgpu::set_last_error_message("invalid arguments");
         return RGPU_ERR_INVALID_ARG;
     }
+    std::lock_guard<std::mutex> lock(g_mu);
     cudaStream_t s = (cudaStream_t)stream;
-    cudaMemsetAsync(loss, 0, 4, s);
-    k_mse<<<1024, 256, 0, s>>>(blurred, target, count, 1.0f / (float)count, loss, grad_blurred);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = cudaSuccess;
+    if (!g_mse.p) {
+        e = g_mse.ensure(sizeof(MseScratch));
+        if (e == cudaSuccess) e = cudaMemsetAsync(g_mse.p, 0, sizeof(MseScratch), s);
+        if (e != cudaSuccess) return fail(e);
+    }
+    k_mse<<<kMseBlocks, kMseThreads, 0, s>>>(blurred, target, count, 1.0f / (float)count, loss, grad_blurred,
+                                             (MseScratch *)g_mse.p);
+    e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     return e == cudaSuccess ? RGPU_OK : fail(e);
 }

@@ -129,3 +129,30 @@ def test_trim_gives_the_scratch_back(gpu):
     assert torch.cuda.mem_get_info()[0] - free >= 1_300_000_000
     again, _ = soft.forward(sc)
     assert torch.equal(again, image)
+
+
+@pytest.mark.parametrize("count", [1, 2, 255, 256, 257, 262143, 262145, 3_000_001])
+def test_loss_is_the_same_every_time(gpu, count):
+    """The loss against float64, and to the bit on every call: its sum does not
+    depend on the order in which blocks finish.  Tolerance: a thread's float sum of
+    at most 12 squares, a factor 1 / count and the result each rounded to 24 bits:
+    14 roundings of 2^-24."""
+    import ctypes as C
+    import resvg_gb300 as R
+    import torch
+    L = R.lib()
+    soft._declare(L)
+    g = torch.Generator(device="cuda").manual_seed(count)
+    a = torch.rand(count, device="cuda", generator=g)
+    b = torch.rand(count, device="cuda", generator=g)
+    out = []
+    for _ in range(4):
+        loss, grad = torch.full((1,), 7.0, device="cuda"), torch.empty_like(a)
+        torch.cuda.synchronize()
+        assert L.rgpu_soft_mse(a.data_ptr(), b.data_ptr(), count, loss.data_ptr(), grad.data_ptr(), None) == 0
+        out.append(float(loss))
+        assert torch.equal(grad, 2.0 * (a - b) * np.float32(1.0 / np.float32(count)))
+    assert len(set(out)) == 1
+    # differences in float32, as the kernel takes them
+    ref = float((a - b).double().pow(2).mean())
+    assert abs(out[0] - ref) <= 14 * 2.0 ** -24 * ref
