@@ -252,17 +252,19 @@ __global__ void k_draw_edges(DrawRec *draws, uint32_t ndraws, const uint32_t *se
     if (dr.valid && e - b < 2) dr.valid = 0;
 }
 
-// The rows of a warp's 32 edges are shared out evenly over its lanes, whatever
-// each edge's height: an edge walking its rows alone waits for one atomic after
-// the other (494 us for the 1024^2 scene's 26 M entries).
+// The rows of a warp's edges (per_warp of them, at most 32) are shared out evenly
+// over its lanes, whatever each edge's height: an edge walking its rows alone
+// waits for one atomic after the other (494 us for the 1024^2 scene's 26 M entries).
+constexpr int kBinThreads = 256;
 template <bool SCATTER>
-__global__ void k_bin(const EdgeRec *edges, const uint32_t *edge_draw, uint32_t nedges, const DrawRec *draws,
-                      const StreamRec *streams, uint32_t *bin_counts, const uint32_t *bin_offsets, uint32_t bin_cap,
-                      uint32_t *err, uint32_t *bins) {
+__global__ void __launch_bounds__(kBinThreads)
+k_bin(const EdgeRec *edges, const uint32_t *edge_draw, uint32_t nedges, uint32_t per_warp, const DrawRec *draws,
+      const StreamRec *streams, uint32_t *bin_counts, const uint32_t *bin_offsets, uint32_t bin_cap, uint32_t *err,
+      uint32_t *bins) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t e = blockIdx.x * blockDim.x + threadIdx.x;
+    const uint32_t e0 = (blockIdx.x * (kBinThreads / 32) + (threadIdx.x >> 5)) * per_warp, e = e0 + lane;
     uint32_t rows = 0, slot = 0, step = 0;  // the edge's rows, the first one's slot, slots per row
-    if (e < nedges) {
+    if (lane < per_warp && e < nedges) {
         const uint32_t d = edge_draw[e];
         const DrawRec &dr = draws[d];
         if (dr.valid) {
@@ -302,11 +304,21 @@ __global__ void k_bin(const EdgeRec *edges, const uint32_t *edge_draw, uint32_t 
             const uint32_t n = atomicAdd(&bin_counts[at], 1u);
             if (SCATTER) {
                 const uint32_t pos = bin_offsets[at] + n;
-                if (pos < bin_cap) bins[pos] = e - lane + k;
+                if (pos < bin_cap) bins[pos] = e0 + k;
                 else atomicOr(err, 1u);
             }
         }
     }
+}
+
+// Few edges are spread thinner, as a warp walks their rows 32 at a time.  Count and
+// emit, us, by 1 / 4 / 8 / 32 edges a warp: 400 edges of 1,000 rows (rules across a
+// 1024^2 canvas) 32 / 91 / 170 / 651, of 2 rows 9 / 9 / 9 / 10; 8,000 of 60 rows 16 /
+// 17 / 22 / 57, of 2 rows 10 / 9 / 10 / 12; 16,000 of 60 rows 26 / 25 / 27 / 60, of 2
+// rows 15 / 10 / 9 / 11; 64,000 of 10 rows 41 / 22 / 19 / 22; 130,000 of 60 rows 138 /
+// 133 / 145 / 160, of 10 rows 72 / 36 / 31 / 30.
+inline uint32_t bin_edges_per_warp(uint32_t nedges) {
+    return nedges <= 8192u ? 1u : nedges <= 32768u ? 4u : nedges <= 131072u ? 8u : 32u;
 }
 
 // ---- exclusive scan (three passes, 1024-element tiles)
@@ -464,12 +476,13 @@ cudaError_t launch_bin(bool scatter, const EdgeRec *edges, const uint32_t *edge_
                        const DrawRec *draws, const StreamRec *streams, uint32_t *bin_counts,
                        const uint32_t *bin_offsets, uint32_t bin_cap, uint32_t *err, uint32_t *bins, cudaStream_t s) {
     if (!nedges) return cudaSuccess;
+    const uint32_t per = bin_edges_per_warp(nedges), blocks = blocks_for(nedges, kBinThreads / 32 * per);
     if (scatter)
-        k_bin<true><<<blocks_for(nedges, 256), 256, 0, s>>>(edges, edge_draw, nedges, draws, streams, bin_counts,
-                                                             bin_offsets, bin_cap, err, bins);
+        k_bin<true><<<blocks, kBinThreads, 0, s>>>(edges, edge_draw, nedges, per, draws, streams, bin_counts,
+                                                   bin_offsets, bin_cap, err, bins);
     else
-        k_bin<false><<<blocks_for(nedges, 256), 256, 0, s>>>(edges, edge_draw, nedges, draws, streams, bin_counts,
-                                                              bin_offsets, bin_cap, err, bins);
+        k_bin<false><<<blocks, kBinThreads, 0, s>>>(edges, edge_draw, nedges, per, draws, streams, bin_counts,
+                                                    bin_offsets, bin_cap, err, bins);
     return cudaGetLastError();
 }
 uint32_t scan_launches(uint64_t n) { return n <= (uint64_t)SCAN_ONE_T * SCAN_ONE_PER ? 1u : 3u; }

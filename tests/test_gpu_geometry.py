@@ -89,3 +89,28 @@ def test_verbs_of_every_kind_match_the_oracle(gpu, oracle_mod, seed):
     got = R.render(t, (1, 0, 0, 1, 0, 0), 120, 110)
     assert got.any()
     assert diff_stats(got, oracle_mod.render(t.view(), (1, 0, 0, 1, 0, 0), 120, 110)) == (0, 0)
+
+
+@pytest.mark.parametrize("edges", [40, 8180, 8200, 32760, 32780, 131060, 131090])
+def test_edges_per_warp_of_the_binning(gpu, oracle_mod, edges):
+    # counts at either side of the lines between 1, 4, 8 and 32 edges a warp, of one
+    # row to the whole canvas
+    w, h = 300, 64
+    g = np.random.default_rng(edges)
+    paths, left = [], edges
+    while left > 0:
+        n = min(left, 1000)
+        y = g.uniform(0.5, h - 0.5, size=(n, 1)) if len(paths) % 2 else np.clip(
+            np.cumsum(g.uniform(-3, 3, size=(n, 1)), axis=0) % h, 0.5, h - 0.5)
+        p = np.concatenate([np.linspace(3, w - 3, n)[:, None] + g.uniform(-1, 1, size=(n, 1)), y], axis=1)
+        paths.append(([A.MOVE] + [A.LINE] * (n - 1) + [A.CLOSE], p.astype(np.float32)))
+        left -= n
+    t = R.Tree(w, h)
+    root = t.add_group(-1, plain_group())
+    for k, (v, p) in enumerate(paths):
+        t.add_path(root, base_path(fill_paint=solid(t, 200 - 40 * (k % 4), 30 + 50 * (k % 3), 90), fill_opacity=0.6,
+                                   fill_rule=A.EVENODD), v, p)
+    t.finalize()
+    got = R.render(t, (1, 0, 0, 1, 0, 0), w, h)
+    assert got.any()
+    assert diff_stats(got, oracle_mod.render(t.view(), (1, 0, 0, 1, 0, 0), w, h)) == (0, 0)
