@@ -479,8 +479,8 @@ __device__ __forceinline__ uint32_t shade_pixel(const PaintRec &pr, const GradRe
 // opacity scale, blend, store.
 __device__ __forceinline__ uint32_t composite_pixel(uint32_t src, uint32_t dst, float opacity, uint32_t blend) {
     // a transparent source over any pixel is that pixel (every byte survives
-    // the way to float and back)
-    if (blend == RGPU_BLEND_DESTINATION || (src == 0u && blend == RGPU_BLEND_SOURCE_OVER)) return dst;
+    // the way to float and back), unless its opacity makes it NaN
+    if (blend == RGPU_BLEND_DESTINATION || (src == 0u && blend == RGPU_BLEND_SOURCE_OVER && isfinite(opacity))) return dst;
     float4 s = unpack_f(src);
     if (opacity != 1.0f) s = make_float4(s.x * opacity, s.y * opacity, s.z * opacity, s.w * opacity);
     return pack_f(blend4(blend, s, unpack_f(dst)));

@@ -58,3 +58,20 @@ def test_gradient_in_a_clip_path(gpu, oracle_mod, kind, aa, rule, opacity):
     ref = oracle_mod.render(t.view(), IDENT, w, h)
     assert ref[..., 3].any()
     assert diff_stats(got, ref) == (0, 0)
+
+
+@pytest.mark.parametrize("opacity", [float("nan"), float("inf"), float("-inf"), -0.5, 2.0, 0.0])
+def test_group_opacity_out_of_range(gpu, oracle_mod, opacity):
+    """A layer whose opacity is no number, infinite or outside [0, 1] composites by
+    the same arithmetic everywhere, its transparent pixels included."""
+    w, h = 70, 20
+    t = R.Tree(w, h)
+    root = t.add_group(-1, plain_group())
+    v, p = rect_path(2, 2, 60, 16)
+    t.add_path(root, base_path(fill_paint=solid(t, 30, 160, 90), fill_opacity=0.8), v, p)
+    g = t.add_group(root, plain_group(opacity=opacity, isolate=1))
+    v, p = rect_path(20.5, 5.3, 20, 9)
+    t.add_path(g, base_path(fill_paint=solid(t, 200, 60, 10), fill_opacity=0.5), v, p)
+    t.finalize()
+    ref = oracle_mod.render(t.view(), IDENT, w, h)
+    assert diff_stats(R.render(t, IDENT, w, h), ref) == (0, 0)
