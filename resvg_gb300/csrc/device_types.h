@@ -88,8 +88,7 @@ struct DrawRec {
     int32_t shift;               // 2: anti-aliased (4x4 supersampling), 0: aliased
     int32_t contained;           // path inside the clip: edges are not clipped
     int32_t sect_l, sect_t, sect_r, sect_b;      // pixel rect coverage may land in
-    int32_t start_y, stop_y, right_clip, super_left;  // scan range in (sub)scanline units
-    uint32_t edge_base, edge_count;
+    int32_t start_y, stop_y;     // scan range in (sub)scanline units
 };
 enum : uint32_t {
     DRAW_EVENODD = 1,

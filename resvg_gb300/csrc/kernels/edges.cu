@@ -5,13 +5,13 @@
 //   k_draw_setup   warp/draw:      transform points, bounds, scan ranges
 //                                  (tiny-skia painter.rs fill_path + scan/path_aa.rs
 //                                  fill_path), segment slots (path.rs PathEdgeIter)
-//   k_edges<false> 8 segments/warp: count line edges
+//   k_edges<false> 1, 4 or 8 segments/warp: count line edges
 //   scan           exclusive prefix sum -> edge offsets
-//   k_edges<true>  8 segments/warp: write line edges (edge_builder.rs)
-//   k_draw_edges   thread/draw:    edge range; paths with < 2 edges are dropped
-//   k_bin<false>   32 edges/warp:   count (row, draw) bin sizes
+//   k_edges<true>  1, 4 or 8 segments/warp: write line edges (edge_builder.rs)
+//   k_draw_edges   thread/draw:    paths with < 2 edges are dropped
+//   k_bin<false>   1 to 32 edges/warp: count (row, draw) bin sizes
 //   scan           -> bin offsets
-//   k_bin<true>    32 edges/warp:   list the edge in its rows' bins
+//   k_bin<true>    1 to 32 edges/warp: list the edge in its rows' bins
 //   k_events       events.cu:      the coverage events of every (row, draw)
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -41,8 +41,6 @@ k_draw_setup(DrawRec *draws, uint32_t ndraws, const uint8_t *scene_verbs, const 
     const uint8_t *verbs = (stroked ? stroke_verbs : scene_verbs) + dr.verb_off;
     const float *pts = (stroked ? stroke_pts : scene_pts) + 2 * (size_t)dr.pt_off;
     dr.valid = 0;
-    dr.edge_base = 0;
-    dr.edge_count = 0;
     auto done = [&]() {
         if (lane == 0) draws[d] = dr;
     };
@@ -101,8 +99,6 @@ k_draw_setup(DrawRec *draws, uint32_t ndraws, const uint8_t *scene_verbs, const 
             int32_t sy0 = iy << 2, sy1 = (iy + ih) << 2;
             if (!contained) { sy0 = max(sy0, 0); sy1 = min(sy1, ch << 2); }
             dr.start_y = sy0; dr.stop_y = sy1;
-            dr.right_clip = cw << 2;
-            dr.super_left = sl << 2;
             dr.valid = 1;
         }
     }
@@ -121,8 +117,6 @@ k_draw_setup(DrawRec *draws, uint32_t ndraws, const uint8_t *scene_verbs, const 
         dr.contained = contained;
         dr.sect_l = 0; dr.sect_t = 0; dr.sect_r = cw; dr.sect_b = ch;
         dr.start_y = y0; dr.stop_y = y1;
-        dr.right_clip = cw;
-        dr.super_left = INT32_MIN;
         dr.valid = 1;
     }
     // ---- segments (PathEdgeIter with implicit close lines), 32 verbs at a
@@ -247,8 +241,6 @@ __global__ void k_draw_edges(DrawRec *draws, uint32_t ndraws, const uint32_t *se
     if (d >= ndraws) return;
     DrawRec &dr = draws[d];
     uint32_t b = seg_offsets[dr.seg_base], e = seg_offsets[dr.seg_base + dr.verb_cnt + 1];
-    dr.edge_base = b;
-    dr.edge_count = e - b;
     if (dr.valid && e - b < 2) dr.valid = 0;
 }
 

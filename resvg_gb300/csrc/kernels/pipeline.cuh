@@ -394,7 +394,7 @@ __device__ __forceinline__ float byte_over_255(float c) {
     return __fmaf_rn(__fmaf_rn(-q, 255.0f, c), kInv255, q);
 }
 
-// shade_pixel for the paints and blend modes off the inline fast path.
+// shade_pixel for the paints and blend modes off the fast path.
 __device__ __forceinline__ uint32_t shade_pixel_slow(const PaintRec &pr, const GradRec *grad, int32_t lx,
                                                          int32_t ly, uint32_t cov, uint32_t dst) {
     const uint32_t blend = pr.blend;
@@ -454,8 +454,7 @@ __device__ __forceinline__ uint32_t shade_pixel_slow(const PaintRec &pr, const G
 }
 
 // Blits one pixel of a fill with coverage `cov` (1..255) onto `dst`: the
-// common lowp source-over case inline, every other paint and blend mode out of
-// line (rare in practice, and kept out of the caller's registers).
+// common lowp source-over case first, then every other paint and blend mode.
 __device__ __forceinline__ uint32_t shade_pixel(const PaintRec &pr, const GradRec *grad, int32_t lx, int32_t ly,
                                                 uint32_t cov, uint32_t dst) {
     if (cov == 255 && (pr.flags & PAINT_MEMSET))

@@ -179,8 +179,7 @@ __device__ __forceinline__ uint32_t scan_row(uint32_t *diff, uint8_t *cov, int32
     return __ballot_sync(0xffffffffu, any != 0u);
 }
 
-// shade_groups for the paints and blend modes off its fast paths (out of line,
-// and out of the caller's registers)
+// shade_groups for the paints and blend modes off its fast paths, one group a step
 __device__ __forceinline__ void shade_groups_slow(uint32_t mask, int bits_sh, const PaintRec *paint, const GradRec *gr,
                                                uint32_t *px, const uint8_t *cov, int32_t lx0, int32_t ly) {
 #pragma unroll 1

@@ -100,14 +100,13 @@ template <> __device__ __forceinline__ float cst<float>(float v) { return v; }
 template <> __device__ __forceinline__ D4 cst<D4>(float v) { return mk(v); }
 
 // Mean of clamp(1 - x, 0, 1) over x running linearly from a to b.
-template <class T>
-__device__ __forceinline__ T mean_right(T a, T b) {
-    if (val(a) > val(b)) { T t = a; a = b; b = t; }
-    if (val(b) <= 0.0f) return cst<T>(1.0f);
-    if (val(a) >= 1.0f) return cst<T>(0.0f);
-    if (val(a) >= 0.0f && val(b) <= 1.0f) return 1.0f - (a + b) * 0.5f;
-    if (val(a) < 0.0f && val(b) <= 1.0f) return 1.0f - (b * b) / ((b - a) * 2.0f);
-    if (val(a) >= 0.0f) return ((1.0f - a) * (1.0f - a)) / ((b - a) * 2.0f);
+__device__ __forceinline__ float mean_right(float a, float b) {
+    if (a > b) { float t = a; a = b; b = t; }
+    if (b <= 0.0f) return 1.0f;
+    if (a >= 1.0f) return 0.0f;
+    if (a >= 0.0f && b <= 1.0f) return 1.0f - (a + b) * 0.5f;
+    if (a < 0.0f && b <= 1.0f) return 1.0f - (b * b) / ((b - a) * 2.0f);
+    if (a >= 0.0f) return ((1.0f - a) * (1.0f - a)) / ((b - a) * 2.0f);
     return (0.5f - a) / (b - a);
 }
 
@@ -314,7 +313,7 @@ k_area(rgpu_soft_batch B, Slice sl, const float2 *verts, uint32_t *overflow) {
         const int xr = first_full(hi, W), xe = min(xr, W);
         Fix prev{0, 0};
         for (int x = first_touched(lo, W); x < xe; x++)
-            add(x, fix40(c.z * mean_right<float>(c.x - (float)x, c.y - (float)x)), prev);
+            add(x, fix40(c.z * mean_right(c.x - (float)x, c.y - (float)x)), prev);
         if (xr < W) add(xr, fix40(c.z), prev);
     });
     if (lane == 0 && total >= (uint32_t)kMaxCross) atomicOr(overflow, 1u);
@@ -954,10 +953,10 @@ uint32_t blocks(uint64_t n, uint32_t per) { return (uint32_t)((n + per - 1) / pe
 // / two groups, us: 500^2 pixels x 4 paths 15.8 / 11.9, x 64 paths 185 / 188; 16
 // scenes of 256 x 512 x 16 385 / 309; but 16 of 256^2 x 64 558 / 757, 1 of 256^2 x 4
 // 9.5 / 11.9.  The lines lie at 160 groups per path and 6,000 in all (640^2 x 64, 200
-// per path, 0.91 .. 1.01; 13 of 117 x 544 x 12, 181 per path, the step 0.98; 256^2 x 16,
-// 128 per path, 0.91 .. 1.39; 256 x 512 x 4, 4,096
-// in all, 1.05; 500^2 x 4, 8,000, 0.75).  The forward composite adds nothing up: one
-// group is never slower there by more than 7%, and up to a third faster.
+// per path, 0.91 .. 1.01; 13 of 117 x 544 x 12, 181 per path, the step 0.98; 256^2 x
+// 16, 128 per path, 0.91 .. 1.39; 256 x 512 x 4, 4,096 in all, 1.05; 500^2 x 4, 8,000,
+// 0.75).  The forward composite adds nothing up: one group is never slower there by
+// more than 7%, and up to a third faster.
 bool wide_strips(const rgpu_soft_batch &b, const Slice &sl) {
     const uint64_t per_scene = (uint64_t)b.height * sl.ng, all = (uint64_t)sl.scenes * sl.rows * sl.ng;
     return sl.ng >= 2 && per_scene >= 160ull * b.paths_per_scene && all >= 6000;
