@@ -13,6 +13,13 @@
 // the events instead of making them again, and neither kernel's code evicts the
 // other's from the instruction caches (one kernel doing both, a warp per row
 // piece, had 9.9 of 13 stalled warps waiting for instructions).
+//
+// What bounds it: issue, at 70% of the slots and 45% of the warps, and the latency
+// of the edge gathers on small scenes: 0.60 ms for 14.2 M binned edges on 1024^2
+// pixels, 4.8 ms for 114.6 M of 128 mixed scenes.  64 registers, as the compiler has
+// it: 80 (3 CTAs per SM) took 2% more of the 1024^2 frame, 95 took 5%.  The gather
+// is free of branches: with one per edge for crossings left of the row a 512^2
+// drawing took 60 us in this kernel for 45.
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "events.cuh"

@@ -75,9 +75,9 @@ cudaError_t launch_raster(uint32_t row_w, uint32_t grid, uint32_t stack_depth, c
                           cudaStream_t s);
 int raster_max_blocks_per_sm(uint32_t row_w);
 // Failure-detection controls of the raster kernel: the try_wait rounds after
-// which a producer/consumer hand-off is declared stuck (0 = the default), and
-// a test hook that withholds the first window of CTA 0 so that wait must run
-// out.  Both apply to launches made afterwards.
+// which a wait for commands is declared stuck (0 = the default), and a test hook
+// by which CTA 0 never asks for its first ones, so that wait must run out.  Both
+// apply to launches made afterwards.
 void raster_set_wait_limit(uint32_t rounds);
 uint32_t raster_wait_limit();
 void raster_set_withhold(bool on);

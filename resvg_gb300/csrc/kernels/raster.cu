@@ -12,12 +12,12 @@
 //
 // What bounds it: instruction issue while enough warps are resident, and a
 // warp's own dependent chain while they are not.  Measured on 1024^2 pixels with
-// 2,000 gradient fills and 500 strokes: 7.0 ms, 3.6 G instructions, 0.42 of the
+// 2,000 gradient fills and 500 strokes: 6.8 ms, 3.6 G instructions, 0.42 of the
 // issue slots (9 warps per SM on average: the rows' costs differ and the last
 // ones run alone).  The kernel before it, with four producer warps per CTA that
 // rasterised spans and eight consumer warps that walked run lists pixel by
 // pixel, took 12.2 ms and issued 6 G; on 256 mixed scenes 29.5 against 84.7 ms
-// (and 9.5 ms in the event kernel).
+// (beside the event kernel: 4.8 ms of it to 17.6 here on 128 of them).
 #include <cuda_runtime.h>
 #include <stdint.h>
 #include "events.cuh"
