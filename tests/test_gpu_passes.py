@@ -138,3 +138,24 @@ def test_failed_allocations_make_smaller_passes(gpu, oracle_mod):
         assert diff_stats(dev.cpu().numpy(), ref) == (0, 0)
         L.rgpu_trim()
         R.render_device(small, IDENT, 64, 16, dev.data_ptr(), 256)
+
+
+def test_more_binned_edges_than_32_bits_number(gpu, oracle_mod):
+    """4.4 G binned edges in 4.4 M slots: 1,000 paths, each a triangle in view and 500
+    contours left of it over all 4,400 rows.  One pass cannot number them."""
+    w, h, n = 64, 4400, 500
+    t = R.Tree(w, h)
+    root = t.add_group(-1, plain_group())
+    g = np.random.default_rng(1)
+    for k in range(1000):
+        x, (y0, y1) = 64 * g.uniform(), np.sort(g.uniform(0, h, 2))
+        xs = g.uniform(-300, -5, n)
+        lo, hi = np.full(n, -1.0), np.full(n, h + 1.0)
+        p = np.concatenate([[x, y0, x + 9, y1, x - 5, y1],
+                            np.stack([xs, lo, xs + 2, lo, xs + 2, hi, xs, hi], 1).ravel()]).astype(np.float32)
+        t.add_path(root, base_path(fill_paint=solid(t, k % 256, 99, 255 - k % 256), fill_opacity=0.5, fill_rule=k & 1),
+                   [A.MOVE, A.LINE, A.LINE, A.CLOSE] + [A.MOVE, A.LINE, A.LINE, A.LINE, A.CLOSE] * n, p)
+    t.finalize()
+    got = R.render(t, IDENT, w, h)
+    assert diff_stats(got, oracle_mod.render(t.view(), IDENT, w, h)) == (0, 0)
+    _lib().rgpu_trim()
