@@ -103,6 +103,10 @@ struct HostBuf {
         if (forced_alloc_failure()) return cudaErrorMemoryAllocation;
         cudaError_t e = cudaMallocHost(&p, want);
         if (e == cudaSuccess) cap = want;
+        else {
+            p = nullptr;
+            cudaGetLastError();
+        }
         return e;
     }
     void release() {
@@ -219,7 +223,8 @@ struct Plan {
 };
 
 // CUDA events around the raster launch of each dependency level (created on
-// first use); the raster time of a render is the sum over its levels.
+// first use); the raster time of a render is the sum over its levels and passes
+// (over the first 16 launches of them).
 struct RasterTimer {
     static constexpr int kPairs = 16;
     cudaEvent_t start[kPairs] = {}, stop[kPairs] = {};
