@@ -346,14 +346,17 @@ int upload(HostBuf &staging, DevBuf &d, const std::vector<T> &v, size_t &stage_o
 }
 
 // The row width of a dependency level's work items (one warp each): the widest
-// that still gives every SM about ten warps.  Wide rows cost least per pixel (a
-// draw is set up once per item), but an item is a serial chain, so too few of
-// them leave the SMs idle: 512 pixels against 128 measured 8.8 against 11.4 ms
-// on 1024^2 pixels (2048 items), 0.55 against 0.50 ms on 512^2 (512 items) and
-// 1.01 against 0.82 ms on 301 x 333.  1024 pixels were never the fastest.
+// that still gives every SM ten and a half warps.  Wide rows cost least per pixel (a
+// draw is set up once per item), but an item is a serial chain, so rows half as
+// wide are faster while all of them run at once, 20 warps per SM.  512 / 256 pixels
+// of 152 SMs: 1024 x 720 (1,440 items of 512 pixels) 1572 / 1519 us, x 768 1609 / 1566,
+// x 800 (1,600) 1591 / 1622, x 900 1693 / 2056, x 1000 1696 / 2287; 1500 x 500 1769 /
+// 1351; with 200 plain fills 1024 x 720 438 / 442, x 800 446 / 475.  256 / 128 pixels:
+// 256 x 768 1353 / 1148, x 1536 1641 / 1520, x 1700 1668 / 1812.  1024 pixels were never
+// the fastest.
 uint32_t pick_row_w(const SceneBuild &sb, uint32_t level, const Tuning &tu, int sms) {
     if (tu.px) return 32 * tu.px;
-    const uint64_t min_items = 10ull * (uint64_t)sms;
+    const uint64_t min_items = 21ull * (uint64_t)sms / 2;
     uint32_t w = 512;
     for (; w > 64; w /= 2) {
         uint64_t n = 0;
